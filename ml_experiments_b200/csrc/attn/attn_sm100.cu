@@ -41,23 +41,6 @@ struct KP {
   int* status;
 };
 
-// Bounded wait shared by all threads of a CTA: once any thread times out (or sees that another CTA has), `*abort_flag`
-// makes every later wait in the CTA return at once, so control flow stays convergent and the kernel terminates. Small, as
-// it is inlined into loops that the instruction cache has to hold.
-__device__ __forceinline__ void cta_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status,
-                                         int code) {
-  uint64_t t0 = 0;
-  for (uint32_t n = 0; !mbar_try_wait(bar, parity); ++n) {
-    if (*abort_flag) return;
-    if ((n & 1023) != 1023) continue;
-    const uint64_t now = globaltimer_ns();
-    if (t0 == 0) t0 = now;
-    const bool late = now - t0 > B200_WAIT_LIMIT_NS;
-    if (late && status) atomicCAS(status, 0, code);
-    if (late || status_poisoned(status)) *abort_flag = 1;
-  }
-}
-
 // ------------------------------------------------------------------------------------------------
 // forward
 // ------------------------------------------------------------------------------------------------

@@ -11,6 +11,7 @@
 #include "fused/fused.h"
 #include "gather/gather_conv.h"
 #include "gather/fused_taps.h"
+#include "gather/tele_band.h"
 #include "fused/norm_act.h"
 #include "gemm/gemm.h"
 #include "mra/mra.h"
@@ -785,30 +786,47 @@ void chk_rows_f32(const Tensor& t, int64_t n, const char* name) {
 }
 
 void tele_fused_fwd(const Tensor& x, const Tensor& freq, const Tensor& phase, const Tensor& kern, const Tensor& expo, Tensor out,
-                    int64_t H, int64_t half, double max_rec) {
+                    int64_t H, int64_t half, double max_rec, const Tensor& status) {
   const c10::cuda::CUDAGuard guard(x.device());
   chk_bf16c(x, "x"); chk_bf16c(out, "out");
   TORCH_CHECK(x.dim() == 3 && out.sizes() == x.sizes() && kern.dim() == 4, "tele_fused: x/out [B,L,C], kern [B,L,H,K]");
   const int B = (int)x.size(0), L = (int)x.size(1), C = (int)x.size(2), K = (int)kern.size(3);
   const int64_t rows = (int64_t)B * L * H;
   chk_rows_f32(freq, rows, "freq"); chk_rows_f32(phase, rows, "phase"); chk_rows_f32(kern, rows * K, "kern"); chk_rows_f32(expo, (int64_t)B * L, "expo");
-  b200::tele_fused_fwd(x.data_ptr(), freq.data_ptr<float>(), phase.data_ptr<float>(), kern.data_ptr<float>(), expo.data_ptr<float>(),
-                       out.data_ptr(), B, L, (int)H, C / (int)H, K, (int)half, (float)max_rec, cur_stream());
+  const float *f = freq.data_ptr<float>(), *ph = phase.data_ptr<float>(), *k = kern.data_ptr<float>(), *e = expo.data_ptr<float>();
+  if (b200::tele_band_takes(x.data_ptr(), out.data_ptr(), B, L, (int)H, C / (int)H, K, (int)half, (float)max_rec, false))
+    b200::tele_band_fwd(x.data_ptr(), f, ph, k, e, out.data_ptr(), B, L, (int)H, C / (int)H, K, (int)half, (float)max_rec,
+                        status.data_ptr<int>(), cur_stream());
+  else
+    b200::tele_fused_fwd(x.data_ptr(), f, ph, k, e, out.data_ptr(), B, L, (int)H, C / (int)H, K, (int)half, (float)max_rec, cur_stream());
 }
 
-void tele_fused_bwd(const Tensor& x, const Tensor& freq, const Tensor& phase, const Tensor& kern, const Tensor& expo, const Tensor& dout,
-                    Tensor dx, Tensor dfreq, Tensor dphase, Tensor dkern, Tensor dexpo_h, int64_t H, int64_t half, double max_rec) {
+// dx: bf16 or fp32 (dx_f32), the others fp32; dexpo_h has a row for each head
+std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> tele_fused_bwd(const Tensor& x, const Tensor& freq, const Tensor& phase, const Tensor& kern,
+                                                                  const Tensor& expo, const Tensor& dout, int64_t H, int64_t half,
+                                                                  double max_rec, bool dx_f32, const Tensor& status) {
   const c10::cuda::CUDAGuard guard(x.device());
   chk_bf16c(x, "x"); chk_bf16c(dout, "dout");
   TORCH_CHECK(x.dim() == 3 && dout.sizes() == x.sizes() && kern.dim() == 4, "tele_fused: x/dout [B,L,C], kern [B,L,H,K]");
   const int B = (int)x.size(0), L = (int)x.size(1), C = (int)x.size(2), K = (int)kern.size(3);
   const int64_t rows = (int64_t)B * L * H;
   chk_rows_f32(freq, rows, "freq"); chk_rows_f32(phase, rows, "phase"); chk_rows_f32(kern, rows * K, "kern"); chk_rows_f32(expo, (int64_t)B * L, "expo");
-  chk_rows_f32(dx, x.numel(), "dx"); chk_rows_f32(dfreq, rows, "dfreq"); chk_rows_f32(dphase, rows, "dphase");
-  chk_rows_f32(dkern, rows * K, "dkern"); chk_rows_f32(dexpo_h, rows, "dexpo_h");
-  b200::tele_fused_bwd(x.data_ptr(), freq.data_ptr<float>(), phase.data_ptr<float>(), kern.data_ptr<float>(), expo.data_ptr<float>(),
-                       dout.data_ptr(), dx.data_ptr<float>(), dfreq.data_ptr<float>(), dphase.data_ptr<float>(), dkern.data_ptr<float>(),
-                       dexpo_h.data_ptr<float>(), B, L, (int)H, C / (int)H, K, (int)half, (float)max_rec, cur_stream());
+  const float *f = freq.data_ptr<float>(), *ph = phase.data_ptr<float>(), *k = kern.data_ptr<float>(), *e = expo.data_ptr<float>();
+  Tensor dfreq = at::empty_like(freq), dphase = at::empty_like(phase), dkern = at::empty_like(kern), dexpo_h = at::empty_like(freq);
+  if (b200::tele_band_takes(x.data_ptr(), dout.data_ptr(), B, L, (int)H, C / (int)H, K, (int)half, (float)max_rec, true)) {
+    Tensor dx = at::empty(x.sizes(), dx_f32 ? x.options().dtype(at::kFloat) : x.options());
+    const int64_t tiles = (int64_t)B * H * ((L + 63) / 64);
+    Tensor plan = at::empty({tiles * 3080}, x.options().dtype(at::kByte));
+    char* queries = (char*)plan.data_ptr();
+    b200::tele_band_bwd(x.data_ptr(), f, ph, k, e, dout.data_ptr(), dx.data_ptr(), dx_f32, dfreq.data_ptr<float>(), dphase.data_ptr<float>(),
+                        dkern.data_ptr<float>(), dexpo_h.data_ptr<float>(), queries + tiles * 3072, queries, B, L, (int)H, C / (int)H, K, (int)half,
+                        (float)max_rec, status.data_ptr<int>(), cur_stream());
+    return {dx, dfreq, dphase, dkern, dexpo_h};
+  }
+  Tensor dx = at::zeros(x.sizes(), x.options().dtype(at::kFloat));
+  b200::tele_fused_bwd(x.data_ptr(), f, ph, k, e, dout.data_ptr(), dx.data_ptr<float>(), dfreq.data_ptr<float>(), dphase.data_ptr<float>(),
+                       dkern.data_ptr<float>(), dexpo_h.data_ptr<float>(), B, L, (int)H, C / (int)H, K, (int)half, (float)max_rec, cur_stream());
+  return {dx_f32 ? dx : dx.to(at::kBFloat16), dfreq, dphase, dkern, dexpo_h};
 }
 
 void alc_fused_fwd(const Tensor& x, const Tensor& half_w, const Tensor& center, const Tensor& kern, Tensor out, int64_t H, int64_t half) {
@@ -1028,8 +1046,8 @@ TORCH_LIBRARY(b200, m) {
   m.def("lincomb3_bwd(Tensor x, Tensor y, Tensor? z, Tensor c, Tensor dout, Tensor(a!) dx, Tensor(b!) dy, Tensor(c!)? dz, Tensor(d!) dc) -> ()");
   m.def("rms_act_fwd(Tensor x, Tensor w, Tensor(a!) y, Tensor(b!) rstd, float eps, int act) -> ()");
   m.def("rms_act_bwd(Tensor x, Tensor w, Tensor rstd, Tensor dy, Tensor? dres, Tensor? dlead, Tensor(a!) dx, Tensor(b!) dw, int act) -> ()");
-  m.def("tele_fused_fwd(Tensor x, Tensor freq, Tensor phase, Tensor kern, Tensor expo, Tensor(a!) out, int H, int half, float max_rec) -> ()");
-  m.def("tele_fused_bwd(Tensor x, Tensor freq, Tensor phase, Tensor kern, Tensor expo, Tensor dout, Tensor(a!) dx, Tensor(b!) dfreq, Tensor(c!) dphase, Tensor(d!) dkern, Tensor(e!) dexpo_h, int H, int half, float max_rec) -> ()");
+  m.def("tele_fused_fwd(Tensor x, Tensor freq, Tensor phase, Tensor kern, Tensor expo, Tensor(a!) out, int H, int half, float max_rec, Tensor(b!) status) -> ()");
+  m.def("tele_fused_bwd(Tensor x, Tensor freq, Tensor phase, Tensor kern, Tensor expo, Tensor dout, int H, int half, float max_rec, bool dx_f32, Tensor(a!) status) -> (Tensor, Tensor, Tensor, Tensor, Tensor)");
   m.def("alc_fused_fwd(Tensor x, Tensor half_w, Tensor center, Tensor kern, Tensor(a!) out, int H, int half) -> ()");
   m.def("alc_fused_bwd(Tensor x, Tensor half_w, Tensor center, Tensor kern, Tensor dout, Tensor(a!) dx, Tensor(b!) dhalf_w, Tensor(c!) dcenter, Tensor(d!) dkern, int H, int half) -> ()");
   m.def("gather_conv_fwd(Tensor x, Tensor pos, Tensor wgt, Tensor(a!) out, int H, float pos_max) -> ()");

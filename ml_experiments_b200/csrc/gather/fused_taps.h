@@ -8,7 +8,7 @@
 //   w = lerp(kern, |rel| / max_rec) * (1 + |rel|/L)^(-expo) * valid,   out += w * bilinear(x, clamp(p, 0, L - 1.001))
 //   freq, phase : fp32 [B][L][H];  kern : fp32 [B][L][H][K];  expo : fp32 [B][L]
 //   backward: dx (fp32, atomics, zero it first), dfreq, dphase [B][L][H], dkern [B][L][H][K], dexpo_h [B][L][H]
-//   (the caller sums dexpo_h over heads).
+//   (the caller sums dexpo_h over heads). Most calls go to tele_band.h instead; these take head_dim 8, little work and very long strides.
 //
 // adaptive local conv (adaptive_local_conv.py:75-169, triton_adaptive_conv.py:81-318):
 //   s in [-half, half]:  r = |s| / half_w,  p = l + center + s,  valid = 0 <= p < L,

@@ -49,11 +49,6 @@ struct SsdParams {
   int* status;
 };
 
-__device__ __forceinline__ void cta_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
-  if (*abort_flag) return;
-  if (!mbar_wait(bar, parity, status, code)) *abort_flag = 1;
-}
-
 // 128 threads: thread t owns time step t of the chunk (rows of G / M / Y / Z) and, for t < N, row t of the state.
 template <int N, int P>
 __global__ void __launch_bounds__(128, (128 + 2 * P) <= 256 ? 2 : 1)

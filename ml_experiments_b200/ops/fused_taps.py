@@ -10,7 +10,7 @@ from __future__ import annotations
 import torch
 
 from .gather_conv import gather_conv_ref
-from .runtime import ops
+from .runtime import ops, status
 
 
 def _lerp_table(table, norm_pos):
@@ -58,7 +58,7 @@ class _Telephone(torch.autograd.Function):
         x16 = x.to(torch.bfloat16).contiguous()
         f, p, k, e = (t.float().contiguous() for t in (freq, phase, kern, expo))
         out = torch.empty_like(x16)
-        ops().tele_fused_fwd(x16, f, p, k, e, out, H, half, max_rec)
+        ops().tele_fused_fwd(x16, f, p, k, e, out, H, half, max_rec, status(x16.device))
         ctx.save_for_backward(x16, f, p, k, e)
         ctx.cfg, ctx.dt = (H, half, max_rec), (x.dtype, freq.dtype, phase.dtype, kern.dtype, expo.dtype)
         return out.to(x.dtype)
@@ -67,12 +67,10 @@ class _Telephone(torch.autograd.Function):
     def backward(ctx, dout):
         x16, f, p, k, e = ctx.saved_tensors
         H, half, max_rec = ctx.cfg
-        dx = torch.zeros(x16.shape, dtype=torch.float32, device=x16.device)
-        df, dp, de_h = torch.empty_like(f), torch.empty_like(p), torch.empty_like(f)
-        dk = torch.empty_like(k)
-        ops().tele_fused_bwd(x16, f, p, k, e, dout.to(torch.bfloat16).contiguous(), dx, df, dp, dk, de_h, H, half, max_rec)
-        de = de_h.view(*f.shape[:2], -1).sum(-1).view(e.shape)
         d = ctx.dt
+        dx, df, dp, dk, de_h = ops().tele_fused_bwd(x16, f, p, k, e, dout.to(torch.bfloat16).contiguous(), H, half, max_rec,
+                                                    d[0] != torch.bfloat16, status(x16.device))
+        de = de_h.view(*f.shape[:2], -1).sum(-1).view(e.shape)
         return dx.to(d[0]), df.to(d[1]), dp.to(d[2]), dk.to(d[3]), de.to(d[4]), None, None, None
 
 

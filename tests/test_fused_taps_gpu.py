@@ -33,6 +33,63 @@ def test_telephone_fused(B, L, H, D, K, half):
         assert _rel(a.grad, b.grad) < 2e-2, (name, _rel(a.grad, b.grad))
 
 
+def _band_inputs(B, L, H, D, K, seed, freq):
+    g = torch.Generator().manual_seed(seed)
+    x = torch.randn(B, L, H * D, generator=g).bfloat16().float()
+    u = torch.rand(B, L, H, generator=g)
+    f = {"wide": u * 15 + 1, "narrow": u * 1.5, "signed": (u - 0.5) * 20, "zero": torch.where(u < 0.3, 0.0, u * 4)}[freq]
+    phase = (torch.rand(B, L, H, generator=g) * 2 - 1) * 16
+    kern = torch.randn(B, L, H, K, generator=g)
+    expo = torch.rand(B, L, 1, generator=g) * 3.5 + 0.5
+    return [t.to("cuda") for t in (x, f, phase, kern, expo)], torch.randn(B, L, H * D, generator=g).bfloat16().float().to("cuda")
+
+
+@pytest.mark.parametrize("B,L,H,D,K,half,freq", [
+    (12, 128, 1, 64, 16, 50, "wide"), (2, 129, 2, 32, 16, 57, "wide"), (1, 191, 4, 16, 64, 59, "signed"), (8, 193, 1, 128, 33, 61, "narrow"),
+    (2, 1000, 3, 64, 16, 54, "zero"), (1, 2051, 2, 128, 64, 51, "signed"), (1, 3001, 2, 32, 16, 55, "wide"), (1, 2500, 1, 64, 2, 117, "narrow"),
+    (1, 2500, 1, 128, 6, 118, "wide"), (2, 1201, 4, 64, 16, 37, "wide"), (1, 300, 2, 64, 16, 4, "wide")])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_telephone_band(B, L, H, D, K, half, freq, dtype):
+    """Edges of the tiles of 128 rows and 64 keys, tables that are no multiple of four, strides below one (several taps on a row), negative
+    and zero ones, results in both precisions; the last one is too little work for the products and is gathered."""
+    from ml_experiments_b200.ops import fused_taps as T
+
+    ins, dout = _band_inputs(B, L, H, D, K, L + D, freq)
+    leaves = [t.clone().to(dtype if i == 0 else t.dtype).requires_grad_(True) for i, t in enumerate(ins)]
+    ref = [t.clone().requires_grad_(True) for t in ins]
+    y = T.telephone_gather(*leaves, H, half, half * 16.0)
+    yr = T.telephone_gather_ref(*ref, H, half, half * 16.0)      # positions in fp32 as here: the same rows are read
+    assert y.dtype == dtype and _rel(y, yr) < 5e-3         # bf16 results
+    y.backward(dout.to(dtype))
+    yr.backward(dout)
+    for i, (name, a, b) in enumerate(zip(("dx", "dfreq", "dphase", "dkern", "dexpo"), leaves, ref)):
+        tol = 5e-3 if i == 0 and dtype == torch.bfloat16 else 2e-4         # results rounded to 2^-9; sums of up to 30000 fp32 products
+        assert _rel(a.grad, b.grad) < tol, (name, _rel(a.grad, b.grad), tol)
+
+
+def test_telephone_band_keeps_what_is_not_finite_where_it_is_sampled():
+    """A row of x (of the gradient) that is not finite reaches the queries that sample it (the rows that it samples) and no others,
+    although products with weights of zero are formed."""
+    from ml_experiments_b200.ops import fused_taps as T
+
+    B, L, H, D, half = 1, 700, 2, 64, 54
+    ins, dout = _band_inputs(B, L, H, D, 16, 5, "wide")
+    ins[0][0, 350, 3] = float("nan")
+    ins[0][0, 200, 70] = float("inf")
+    dout[0, 333, 5] = float("nan")
+    leaves, ref = [t.clone().requires_grad_(True) for t in ins], [t.clone().requires_grad_(True) for t in ins]
+    y = T.telephone_gather(*leaves, H, half, half * 16.0)
+    yr = T.telephone_gather_ref(*ref, H, half, half * 16.0)
+    bad = yr.isfinite().logical_not()
+    assert bad.any() and torch.equal(y.isfinite().logical_not(), bad)
+    assert _rel(y[~bad], yr[~bad]) < 5e-3
+    y.backward(dout)
+    yr.backward(dout)
+    inner = slice(2, L - 2)                                # taps outside are moved to the ends in the restatement, with weight zero
+    bad = ref[0].grad[:, inner].isfinite().logical_not()
+    assert bad.any() and torch.equal(leaves[0].grad[:, inner].isfinite().logical_not(), bad)
+
+
 @pytest.mark.parametrize("B,L,H,D,K,half", [(2, 300, 4, 64, 64, 29), (1, 1000, 2, 16, 16, 9), (2, 130, 3, 128, 8, 3), (1, 257, 8, 8, 64, 12)])
 def test_adaptive_local_fused(B, L, H, D, K, half):
     from ml_experiments_b200.ops import fused_taps as T
