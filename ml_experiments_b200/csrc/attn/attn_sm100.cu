@@ -138,7 +138,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   constexpr uint32_t O_COL = 0, P_COL = 2 * D, S_COL = 2 * D + 128, TMEM_COLS = 512;
 
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* smem = smem_raw + (-smem_u32(smem_raw) & 1023u);
   uint8_t* sQ = smem;
   uint8_t* sKV = sQ + 2 * F::Q_BYTES;
   uint64_t* bars = reinterpret_cast<uint64_t*>(sKV + NST * F::KV_BYTES);
@@ -538,7 +538,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   constexpr uint32_t TMEM_COLS = 512;
 
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* smem = smem_raw + (-smem_u32(smem_raw) & 1023u);
   uint8_t* sK = smem;
   uint8_t* sV = sK + KV_BYTES;
   constexpr int NQB = 3;              // Q / dO buffers
