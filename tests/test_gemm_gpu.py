@@ -93,6 +93,40 @@ def test_gemm_fp8(a_mn, b_mn):
     assert _rel_err(out, 0.25 * ref) < 2e-3
 
 
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, False)])
+@pytest.mark.parametrize("m,n,k,batch", [(8193, 2312, 1096, None), (16384 + 128, 776, 1608, None), (640, 1032, 1032, 33)])
+def test_gemm_by_pairs(a_mn, b_mn, m, n, k, batch):
+    """Products large enough for pairs of CTAs on tiles of 256 x 256: a last tile of one row, of one CTA only, of a few columns; a K that
+    is no multiple of a stage; batches; every epilogue."""
+    from ml_experiments_b200.ops import gemm as G
+
+    m = (m + 7) // 8 * 8 if a_mn else m          # (rows of 16-byte multiples)
+    assert 2 * m * n * k * (batch or 1) >= 4e10
+    torch.manual_seed(7)
+    pre = () if batch is None else (batch,)
+    a = torch.randn(*pre, *((k, m) if a_mn else (m, k)), device="cuda", dtype=torch.bfloat16)
+    b = torch.randn(*pre, *((k, n) if b_mn else (n, k)), device="cuda", dtype=torch.bfloat16)
+    aux = torch.randn(*pre, m, n, device="cuda", dtype=torch.bfloat16).square()
+    ref = _ref(a, b, a_mn, b_mn)
+    kw = dict(a_mn=a_mn, b_mn=b_mn)
+    assert _rel_err(G.gemm(a, b, **kw), ref) < 6e-3
+    assert _rel_err(G.gemm(a, b, out_dtype=torch.float32, **kw), ref) < 2e-3
+    assert _rel_err(G.gemm(a, b, epilogue=G.EPI_RELU2, alpha=0.05, **kw), torch.relu(ref * 0.05) ** 2) < 1e-2
+    assert _rel_err(G.gemm(a, b, epilogue=G.EPI_AXPBY, aux=aux, alpha=0.5, beta=-2.0, **kw), 0.5 * ref - 2.0 * aux.float()) < 6e-3
+    assert _rel_err(G.gemm(a, b, epilogue=G.EPI_RELU2_BWD, aux=aux, **kw), ref * 2 * aux.float().sqrt()) < 1e-2
+
+
+def test_gemm_fp8_by_pairs():
+    from ml_experiments_b200.ops.gemm import gemm
+
+    torch.manual_seed(8)
+    m, n, k = 3000, 5008, 1424
+    a = torch.randn(m, k, device="cuda").to(torch.float8_e4m3fn)
+    for b_mn in (False, True):
+        b = torch.randn((k, n) if b_mn else (n, k), device="cuda").to(torch.float8_e5m2 if b_mn else torch.float8_e4m3fn)
+        assert _rel_err(gemm(a, b, b_mn=b_mn, out_dtype=torch.float32, alpha=0.25), 0.25 * _ref(a, b, False, b_mn)) < 2e-3
+
+
 def test_output_aliasing_an_operand_is_refused():
     """In-place products are a timing-dependent race between CTAs (one stores a tile of the operand another still
     reads); the front end rejects them instead of returning numbers that are right most of the time."""

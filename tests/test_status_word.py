@@ -17,7 +17,7 @@ def test_no_thread_returns_by_its_own_read_of_the_status_word():
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("op", ["attn_fwd", "attn_bwd", "gemm", "ssd_fwd"])
+@pytest.mark.parametrize("op", ["attn_fwd", "attn_bwd", "gemm", "gemm_pair", "ssd_fwd"])
 def test_kernels_leave_at_once_while_the_word_is_set(op):
     from ml_experiments_b200.ops import attention as A
     from ml_experiments_b200.ops.runtime import check_status, ops, status
@@ -37,8 +37,9 @@ def test_kernels_leave_at_once_while_the_word_is_set(op):
             outs = [mark(t, h, d, dt=torch.float32), mark(t, h, d), mark(t, h, d)]
             delta = torch.empty(h, t, device="cuda")
             call = lambda: ops().attn_bwd(q, k, v, o, d_o, lse, delta, *outs, ds, de, 0.12, 0, st)  # noqa: E731
-    elif op == "gemm":
-        a, b, outs = bf(256, 128), bf(384, 128), [mark(256, 384)]
+    elif op.startswith("gemm"):
+        m, k = (256, 128) if op == "gemm" else (40960, 2048)         # by pairs of CTAs, whose both must leave
+        a, b, outs = bf(m, k), bf(384, k), [mark(m, 384)]
         call = lambda: ops().gemm(a, b, outs[0], None, False, False, 0, 1.0, 0.0, 1, False, st)  # noqa: E731
     else:
         x, B, C = bf(1, 256, 2, 64), bf(1, 256, 2, 64), bf(1, 256, 2, 64)
