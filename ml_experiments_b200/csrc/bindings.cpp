@@ -15,6 +15,7 @@
 #include "fused/norm_act.h"
 #include "gemm/gemm.h"
 #include "mra/mra.h"
+#include "scan/s6_mixer.h"
 #include "scan/s6_scan.h"
 #include "scan/jacobi.h"
 #include "scan/ssd.h"
@@ -632,6 +633,57 @@ void s6_scan_bwd(const Tensor& u, const Tensor& delta, const c10::optional<Tenso
 }
 
 
+// conv weight, conv bias, A_log, D and step bias of an S6 mixer, dense, fp32 or bf16
+b200::S6Tensors s6_tensors(at::TensorList t, int64_t C) {
+  TORCH_CHECK(t.size() == 5, "s6: five parameters");
+  static const int64_t per[5] = {4, 1, 16, 1, 1};
+  b200::S6Tensors o;
+  for (int i = 0; i < 5; ++i) {
+    TORCH_CHECK(t[i].is_cuda() && t[i].is_contiguous() && t[i].numel() == C * per[i] &&
+                (t[i].scalar_type() == at::kFloat || t[i].scalar_type() == at::kBFloat16), "s6: parameter ", i, " must be dense fp32 or bf16 of its size");
+    o.ptr[i] = t[i].data_ptr();
+    o.bf16[i] = t[i].scalar_type() == at::kBFloat16;
+  }
+  return o;
+}
+Tensor s6_params(at::TensorList params) {
+  TORCH_CHECK(params.size() == 5, "s6: five parameters");
+  const c10::cuda::CUDAGuard guard(params[0].device());
+  const int64_t C = params[3].numel();
+  Tensor packed = at::empty({23 * C}, params[0].options().dtype(at::kFloat));
+  b200::s6_params(s6_tensors(params, C), packed.data_ptr<float>(), (int)C, cur_stream());
+  return packed;
+}
+std::vector<Tensor> s6_param_grads(at::TensorList params, const Tensor& grads, const Tensor& packed) {
+  TORCH_CHECK(params.size() == 5, "s6: five parameters");
+  const c10::cuda::CUDAGuard guard(grads.device());
+  const int64_t C = params[3].numel();
+  for (const Tensor& t : {grads, packed})
+    TORCH_CHECK(t.is_cuda() && t.is_contiguous() && t.scalar_type() == at::kFloat && t.numel() == 23 * C, "s6: gradients and packed parameters: fp32 [23 C]");
+  std::vector<Tensor> out;
+  for (const Tensor& p : params) out.push_back(at::empty_like(p));
+  b200::s6_param_grads(s6_tensors(out, C), grads.data_ptr<float>(), packed.data_ptr<float>(), (int)C, cur_stream());
+  return out;
+}
+void chk_dbc(const Tensor& t, const char* name) {
+  chk_bf16c(t, name);
+  TORCH_CHECK(t.dim() == 2 && t.size(1) >= 32 && t.size(1) % 8 == 0 && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0, name, ": bf16 [rows, 8 n + 32], 16-byte aligned");
+}
+Tensor s6_split_bc(const Tensor& dbc) {
+  const c10::cuda::CUDAGuard guard(dbc.device());
+  chk_dbc(dbc, "dbc");
+  Tensor bc = at::empty({2, dbc.size(0), 16}, dbc.options().dtype(at::kFloat));
+  b200::s6_split_bc(dbc.data_ptr(), bc.data_ptr<float>(), dbc.size(0), (int)dbc.size(1), cur_stream());
+  return bc;
+}
+void s6_join_bc(const Tensor& parts, Tensor ddbc) {
+  const c10::cuda::CUDAGuard guard(ddbc.device());
+  chk_dbc(ddbc, "ddbc");
+  TORCH_CHECK(parts.is_cuda() && parts.scalar_type() == at::kFloat && parts.is_contiguous() && parts.dim() == 5 && parts.size(0) == 2 && parts.size(4) == 16 &&
+              parts.size(1) * parts.size(3) == ddbc.size(0), "parts: fp32 [2, batch, blocks, L, 16]");
+  b200::s6_join_bc(parts.data_ptr<float>(), ddbc.data_ptr(), (int)parts.size(1), (int)parts.size(2), (int)parts.size(3), (int)ddbc.size(1), cur_stream());
+}
+
 void causal_conv1d_silu_fwd(const Tensor& x, const Tensor& w, const c10::optional<Tensor>& bias, Tensor y) {
   const c10::cuda::CUDAGuard guard(x.device());
   TORCH_CHECK(x.dim() == 3 && x.scalar_type() == at::kBFloat16 && x.stride(2) == 1 && x.stride(0) == x.size(1) * x.stride(1), "x: bf16 [B, L, C] (channel slice allowed)");
@@ -956,14 +1008,18 @@ void lincomb3_bwd(const Tensor& x, const Tensor& y, const c10::optional<Tensor>&
                      dy.data_ptr(), dz.has_value() ? dz->data_ptr() : nullptr, dc.data_ptr<float>(), n, cur_stream());
 }
 
+void chk_norm_weight(const Tensor& w, int64_t C) {
+  TORCH_CHECK(w.is_cuda() && w.is_contiguous() && w.numel() == C && (w.scalar_type() == at::kFloat || w.scalar_type() == at::kBFloat16), "weight: dense fp32 or bf16 [C]");
+}
+
 void rms_act_fwd(const Tensor& x, const Tensor& w, Tensor y, Tensor rstd, double eps, int64_t act) {
   const c10::cuda::CUDAGuard guard(x.device());
   const bool xb = norm_io_bf16(x, "x"), yb = norm_io_bf16(y, "y");
   const int C = (int)x.size(-1);
   const int64_t R = x.numel() / C;
   TORCH_CHECK(y.numel() == x.numel(), "y: x's shape");
-  chk_rows_f32(w, C, "weight"); chk_rows_f32(rstd, R, "rstd");
-  b200::rms_act_fwd(x.data_ptr(), xb, w.data_ptr<float>(), y.data_ptr(), yb, rstd.data_ptr<float>(), R, C, (float)eps, (int)act, cur_stream());
+  chk_norm_weight(w, C); chk_rows_f32(rstd, R, "rstd");
+  b200::rms_act_fwd(x.data_ptr(), xb, w.data_ptr(), w.scalar_type() == at::kBFloat16, y.data_ptr(), yb, rstd.data_ptr<float>(), R, C, (float)eps, (int)act, cur_stream());
 }
 
 void rms_act_bwd(const Tensor& x, const Tensor& w, const Tensor& rstd, const Tensor& dy, const c10::optional<Tensor>& dres,
@@ -973,7 +1029,7 @@ void rms_act_bwd(const Tensor& x, const Tensor& w, const Tensor& rstd, const Ten
   TORCH_CHECK(norm_io_bf16(dx, "dx") == xb && dx.numel() == x.numel() && dy.numel() == x.numel(), "dx: x's dtype and shape; dy: x's shape");
   const int C = (int)x.size(-1);
   const int64_t R = x.numel() / C;
-  chk_rows_f32(w, C, "weight"); chk_rows_f32(rstd, R, "rstd"); chk_rows_f32(dw, C, "dw");
+  chk_norm_weight(w, C); chk_rows_f32(rstd, R, "rstd"); chk_rows_f32(dw, C, "dw");
   const void* res = nullptr;
   if (dres.has_value()) {
     TORCH_CHECK(dres->is_cuda() && dres->is_contiguous() && dres->scalar_type() == x.scalar_type() && dres->numel() == x.numel(),
@@ -988,7 +1044,7 @@ void rms_act_bwd(const Tensor& x, const Tensor& w, const Tensor& rstd, const Ten
     lead_p = dlead->data_ptr();
     lead = (int)dlead->size(-1);
   }
-  b200::rms_act_bwd(x.data_ptr(), xb, w.data_ptr<float>(), rstd.data_ptr<float>(), dy.data_ptr(), gb, res, lead_p, lead, dx.data_ptr(),
+  b200::rms_act_bwd(x.data_ptr(), xb, w.data_ptr(), w.scalar_type() == at::kBFloat16, rstd.data_ptr<float>(), dy.data_ptr(), gb, res, lead_p, lead, dx.data_ptr(),
                     dw.data_ptr<float>(), R, C, (int)act, cur_stream());
 }
 
@@ -1036,6 +1092,10 @@ TORCH_LIBRARY(b200, m) {
   m.def("ssd_fwd(Tensor x, Tensor B, Tensor C, Tensor log_a, Tensor g_off, Tensor g_diag, Tensor(a!) y, Tensor? init_state, Tensor(b!)? final_state, Tensor(c!) status, Tensor(d!)? chunk_states=None) -> ()");
   m.def("s6_scan_fwd(Tensor u, Tensor delta, Tensor? delta_bias, bool softplus, Tensor A, Tensor Bm, Tensor Cm, Tensor? Dv, Tensor? z, Tensor(a!)? y_pre, Tensor(b!) out, Tensor(c!)? state) -> ()");
   m.def("s6_scan_bwd(Tensor u, Tensor delta, Tensor? delta_bias, bool softplus, Tensor A, Tensor Bm, Tensor Cm, Tensor? Dv, Tensor? z, Tensor? y_pre, Tensor dout, Tensor state, Tensor(a!) du, Tensor(b!) ddelta, Tensor(c!) dA, Tensor(d!) dB_part, Tensor(e!) dC_part, Tensor(f!)? dD, Tensor(g!)? dz, Tensor(h!)? ddelta_bias) -> ()");
+  m.def("s6_params(Tensor[] params) -> Tensor");
+  m.def("s6_param_grads(Tensor[] params, Tensor grads, Tensor packed) -> Tensor[]");
+  m.def("s6_split_bc(Tensor dbc) -> Tensor");
+  m.def("s6_join_bc(Tensor parts, Tensor(a!) ddbc) -> ()");
   m.def("causal_conv1d_silu_fwd(Tensor x, Tensor w, Tensor? bias, Tensor(a!) y) -> ()");
   m.def("causal_conv1d_silu_bwd(Tensor x, Tensor w, Tensor? bias, Tensor dy, Tensor(a!) dx, Tensor(b!) dw, Tensor(c!)? dbias) -> ()");
   m.def("norm_rope_fwd(Tensor x, Tensor f1, Tensor f2, Tensor(a!) y, Tensor(b!) rstd, float eps) -> ()");
@@ -1102,6 +1162,10 @@ TORCH_LIBRARY_IMPL(b200, CUDA, m) {
   m.impl("jacobi_fwd", &jacobi_fwd);
   m.impl("jacobi_bwd", &jacobi_bwd);
   m.impl("s6_scan_fwd", &s6_scan_fwd);
+  m.impl("s6_params", &s6_params);
+  m.impl("s6_param_grads", &s6_param_grads);
+  m.impl("s6_split_bc", &s6_split_bc);
+  m.impl("s6_join_bc", &s6_join_bc);
   m.impl("s6_scan_bwd", &s6_scan_bwd);
   m.impl("causal_conv1d_silu_fwd", &causal_conv1d_silu_fwd);
   m.impl("causal_conv1d_silu_bwd", &causal_conv1d_silu_bwd);

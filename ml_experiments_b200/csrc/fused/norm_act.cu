@@ -15,6 +15,10 @@ using bf16 = __nv_bfloat16;
 template <typename T> __device__ __forceinline__ float ldf(const T* p, long long i);
 template <> __device__ __forceinline__ float ldf<float>(const float* p, long long i) { return p[i]; }
 template <> __device__ __forceinline__ float ldf<bf16>(const bf16* p, long long i) { return __bfloat162float(p[i]); }
+// weight c, fp32 or bf16
+__device__ __forceinline__ float ldw(const void* w, bool wb, int c) {
+  return wb ? __bfloat162float(reinterpret_cast<const bf16*>(w)[c]) : reinterpret_cast<const float*>(w)[c];
+}
 template <typename T> __device__ __forceinline__ void stf(T* p, long long i, float v);
 template <> __device__ __forceinline__ void stf<float>(float* p, long long i, float v) { p[i] = v; }
 template <> __device__ __forceinline__ void stf<bf16>(bf16* p, long long i, float v) { p[i] = __float2bfloat16(v); }
@@ -51,7 +55,7 @@ __device__ __forceinline__ float act_grad(float u) {
 
 template <typename TI, typename TO, int ACT>
 __global__ void __launch_bounds__(256)
-rms_act_fwd_kernel(const TI* __restrict__ x, const float* __restrict__ w, TO* __restrict__ y, float* __restrict__ rstd,
+rms_act_fwd_kernel(const TI* __restrict__ x, const void* __restrict__ w, bool wb, TO* __restrict__ y, float* __restrict__ rstd,
                    long long R, int C, float eps) {
   const int lane = threadIdx.x & 31;
   const long long warps = (long long)gridDim.x * 8;
@@ -64,13 +68,61 @@ rms_act_fwd_kernel(const TI* __restrict__ x, const float* __restrict__ w, TO* __
     }
     const float rs = rsqrtf(warp_sum(ss) / (float)C + eps);
     if (lane == 0) rstd[row] = rs;
-    for (int c = lane; c < C; c += 32) stf(y, base + c, act_fwd<ACT>(w[c] * ldf(x, base + c) * rs));
+    for (int c = lane; c < C; c += 32) stf(y, base + c, act_fwd<ACT>(ldw(w, wb, c) * ldf(x, base + c) * rs));
+  }
+}
+
+// Forward for bf16 rows of 256 * VPL columns: a lane moves groups of 8 columns with 16-byte accesses and keeps its part of the row, which is
+// read once, and of the weights, which are read once per warp. Bound: memory, one read and one write of the rows.
+// 32768 x 1024: 22 us (31 us with a column per lane and access and two reads).
+template <int VPL, int ACT>
+__global__ void __launch_bounds__(256)
+rms_act_fwd_vec_kernel(const bf16* __restrict__ x, const void* __restrict__ w, bool wb, bf16* __restrict__ y, float* __restrict__ rstd, long long R,
+                       float eps) {
+  constexpr int C = VPL * 256;
+  const int lane = threadIdx.x & 31;
+  float wv[VPL][8];
+#pragma unroll
+  for (int j = 0; j < VPL; ++j)
+#pragma unroll
+    for (int e = 0; e < 8; ++e) wv[j][e] = ldw(w, wb, (j * 32 + lane) * 8 + e);
+  const long long warps = (long long)gridDim.x * 8;
+  for (long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); row < R; row += warps) {
+    const uint4* src = reinterpret_cast<const uint4*>(x + row * C) + lane;
+    uint4* dst = reinterpret_cast<uint4*>(y + row * C) + lane;
+    uint4 u[VPL];
+#pragma unroll
+    for (int j = 0; j < VPL; ++j) u[j] = src[j * 32];
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < VPL; ++j) {
+      const uint32_t v[4] = {u[j].x, u[j].y, u[j].z, u[j].w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float a = __uint_as_float(v[e] << 16), b = __uint_as_float(v[e] & 0xffff0000u);
+        ss = fmaf(a, a, fmaf(b, b, ss));
+      }
+    }
+    const float rs = rsqrtf(warp_sum(ss) / (float)C + eps);
+    if (lane == 0) rstd[row] = rs;
+#pragma unroll
+    for (int j = 0; j < VPL; ++j) {
+      const uint32_t v[4] = {u[j].x, u[j].y, u[j].z, u[j].w};
+      uint32_t o[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float a = __uint_as_float(v[e] << 16), b = __uint_as_float(v[e] & 0xffff0000u);
+        const __nv_bfloat162 h = __floats2bfloat162_rn(act_fwd<ACT>(wv[j][2 * e] * a * rs), act_fwd<ACT>(wv[j][2 * e + 1] * b * rs));
+        o[e] = *reinterpret_cast<const uint32_t*>(&h);
+      }
+      dst[j * 32] = make_uint4(o[0], o[1], o[2], o[3]);
+    }
   }
 }
 
 template <typename TI, typename TO, int ACT>
 __global__ void __launch_bounds__(256)
-rms_act_bwd_kernel(const TI* __restrict__ x, const float* __restrict__ w, const float* __restrict__ rstd,
+rms_act_bwd_kernel(const TI* __restrict__ x, const void* __restrict__ w, bool wb, const float* __restrict__ rstd,
                    const TO* __restrict__ dy, const TI* __restrict__ dres, const TO* __restrict__ dlead, int lead,
                    TI* __restrict__ dx, float* __restrict__ dw, long long R, int C) {
   extern __shared__ float s_dw[];  // [C]
@@ -90,21 +142,21 @@ rms_act_bwd_kernel(const TI* __restrict__ x, const float* __restrict__ w, const 
     for (int i = 0; i < 8; ++i) {  // the first 256 columns accumulate dw in registers
       const int c = lane + 32 * i;
       if (c < C) {
-        const float xh = ldf(x, base + c) * rs, wc = w[c];
+        const float xh = ldf(x, base + c) * rs, wc = ldw(w, wb, c);
         const float g = gin(c) * act_grad<ACT>(wc * xh);
         dot += g * wc * xh;
         acc[i] += g * xh;
       }
     }
     for (int c = lane + 256; c < C; c += 32) {
-      const float xh = ldf(x, base + c) * rs, wc = w[c];
+      const float xh = ldf(x, base + c) * rs, wc = ldw(w, wb, c);
       const float g = gin(c) * act_grad<ACT>(wc * xh);
       dot += g * wc * xh;
       atomicAdd(&s_dw[c], g * xh);
     }
     dot = warp_sum(dot) * invC;
     for (int c = lane; c < C; c += 32) {
-      const float xh = ldf(x, base + c) * rs, wc = w[c];
+      const float xh = ldf(x, base + c) * rs, wc = ldw(w, wb, c);
       const float g = gin(c) * act_grad<ACT>(wc * xh);
       stf(dx, base + c, rs * (g * wc - xh * dot) + (dres ? ldf(dres, base + c) : 0.f));
     }
@@ -152,7 +204,7 @@ __device__ __forceinline__ uint4 ldg128_again(const void* p) {
 // read twice (the second time from L1): holding a row between the passes costs the registers of the second resident block.
 template <int VPL, int ACT>
 __global__ void __launch_bounds__(256, 2)
-rms_act_bwd_vec_kernel(const bf16* __restrict__ x, const float* __restrict__ w, const float* __restrict__ rstd,
+rms_act_bwd_vec_kernel(const bf16* __restrict__ x, const void* __restrict__ w, bool wb, const float* __restrict__ rstd,
                        const bf16* __restrict__ dy, const bf16* __restrict__ dres, const bf16* __restrict__ dlead, int lead,
                        bf16* __restrict__ dx, float* __restrict__ dw, long long R) {
   constexpr int C = VPL * 256;
@@ -160,7 +212,7 @@ rms_act_bwd_vec_kernel(const bf16* __restrict__ x, const float* __restrict__ w, 
   __shared__ __align__(16) float s_w[C];
   for (int c = threadIdx.x; c < C; c += 256) {
     s_dw[c] = 0.f;
-    s_w[c] = w[c];
+    s_w[c] = ldw(w, wb, c);
   }
   __syncthreads();
   const int lane = threadIdx.x & 31;
@@ -268,17 +320,30 @@ int grid_for(long long R) {
   else { using TI_ = float; using TO_ = float; __VA_ARGS__; }
 }  // namespace
 
-void rms_act_fwd(const void* x, bool x_bf16, const float* w, void* y, bool y_bf16, float* rstd, long long R, int C, float eps,
+void rms_act_fwd(const void* x, bool x_bf16, const void* w, bool w_bf16, void* y, bool y_bf16, float* rstd, long long R, int C, float eps,
                  int act, cudaStream_t s) {
   if (C < 1 || C > 4096) throw std::runtime_error("rms_act: row length must be in [1, 4096]");
   if (R == 0) return;
+  const bool even = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
+  if (x_bf16 && y_bf16 && even && C % 256 == 0 && C <= 1024) {
+#define RMS_VEC(VPL_) DISPATCH_ACT(act, rms_act_fwd_vec_kernel<VPL_, ACT_><<<grid_for(R), 256, 0, s>>>((const bf16*)x, w, w_bf16, (bf16*)y, rstd, R, eps))
+    switch (C / 256) {
+      case 1: RMS_VEC(1); break;
+      case 2: RMS_VEC(2); break;
+      case 3: RMS_VEC(3); break;
+      default: RMS_VEC(4); break;
+    }
+#undef RMS_VEC
+    chk("rms_act_fwd");
+    return;
+  }
   DISPATCH_ACT(act, DISPATCH_IO(x_bf16, y_bf16, {
-    rms_act_fwd_kernel<TI_, TO_, ACT_><<<grid_for(R), 256, 0, s>>>((const TI_*)x, w, (TO_*)y, rstd, R, C, eps);
+    rms_act_fwd_kernel<TI_, TO_, ACT_><<<grid_for(R), 256, 0, s>>>((const TI_*)x, w, w_bf16, (TO_*)y, rstd, R, C, eps);
   }));
   chk("rms_act_fwd");
 }
 
-void rms_act_bwd(const void* x, bool x_bf16, const float* w, const float* rstd, const void* dy, bool dy_bf16,
+void rms_act_bwd(const void* x, bool x_bf16, const void* w, bool w_bf16, const float* rstd, const void* dy, bool dy_bf16,
                  const void* dres, const void* dlead, int lead, void* dx, float* dw, long long R, int C, int act,
                  cudaStream_t s) {
   if (dlead == nullptr) lead = 0;
@@ -286,11 +351,11 @@ void rms_act_bwd(const void* x, bool x_bf16, const float* w, const float* rstd, 
   if (C < 1 || C > 4096) throw std::runtime_error("rms_act: row length must be in [1, 4096]");
   if (R == 0) return;
   const bool aligned = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(dx) |
-                         reinterpret_cast<uintptr_t>(dres) | reinterpret_cast<uintptr_t>(w)) & 15) == 0;
+                         reinterpret_cast<uintptr_t>(dres)) & 15) == 0;
   if (x_bf16 && dy_bf16 && aligned && C % 256 == 0 && C <= 1024) {
     const int grid = (int)std::min<long long>((R + 7) / 8, 148LL * 4);
 #define RMS_VEC(VPL_)                                                                                                  \
-  DISPATCH_ACT(act, rms_act_bwd_vec_kernel<VPL_, ACT_><<<grid, 256, 0, s>>>((const bf16*)x, w, rstd, (const bf16*)dy,  \
+  DISPATCH_ACT(act, rms_act_bwd_vec_kernel<VPL_, ACT_><<<grid, 256, 0, s>>>((const bf16*)x, w, w_bf16, rstd, (const bf16*)dy,  \
                                                                              (const bf16*)dres, (const bf16*)dlead, lead,    \
                                                                              (bf16*)dx, dw, R))
     switch (C / 256) {
@@ -304,7 +369,7 @@ void rms_act_bwd(const void* x, bool x_bf16, const float* w, const float* rstd, 
     return;
   }
   DISPATCH_ACT(act, DISPATCH_IO(x_bf16, dy_bf16, {
-    rms_act_bwd_kernel<TI_, TO_, ACT_><<<grid_for(R), 256, (size_t)C * sizeof(float), s>>>((const TI_*)x, w, rstd, (const TO_*)dy, (const TI_*)dres, (const TO_*)dlead, lead, (TI_*)dx, dw, R, C);
+    rms_act_bwd_kernel<TI_, TO_, ACT_><<<grid_for(R), 256, (size_t)C * sizeof(float), s>>>((const TI_*)x, w, w_bf16, rstd, (const TO_*)dy, (const TI_*)dres, (const TO_*)dlead, lead, (TI_*)dx, dw, R, C);
   }));
   chk("rms_act_bwd");
 }

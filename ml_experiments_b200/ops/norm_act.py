@@ -21,26 +21,32 @@ def rms_norm_act_ref(x, weight, eps: float = 1e-6, act: str = "none", out_dtype=
     return y.to(out_dtype or x.dtype)
 
 
+def _weight(w):
+    """The weight as the kernels read it: dense, fp32 or bf16."""
+    w = w.detach()
+    return (w if w.dtype in (torch.float32, torch.bfloat16) else w.float()).contiguous()
+
+
 class _RmsAct(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, eps, act, out_dtype):
         xc = x.contiguous()
-        w32 = weight.detach().float().contiguous()
+        w = _weight(weight)
         y = torch.empty(xc.shape, dtype=out_dtype, device=x.device)
         rstd = torch.empty(xc.numel() // xc.shape[-1], dtype=torch.float32, device=x.device)
-        ops().rms_act_fwd(xc, w32, y, rstd, eps, act)
-        ctx.save_for_backward(xc, w32, rstd)
+        ops().rms_act_fwd(xc, w, y, rstd, eps, act)
+        ctx.save_for_backward(xc, w, rstd)
         ctx.act, ctx.wdtype = act, weight.dtype
         return y
 
     @staticmethod
     def backward(ctx, dy):
-        xc, w32, rstd = ctx.saved_tensors
+        xc, w, rstd = ctx.saved_tensors
         if dy.dtype not in (torch.bfloat16, torch.float32):
             dy = dy.float()
         dx = torch.empty_like(xc)
-        dw = torch.zeros_like(w32)
-        ops().rms_act_bwd(xc, w32, rstd, dy.contiguous(), None, None, dx, dw, ctx.act)
+        dw = torch.zeros(w.shape, dtype=torch.float32, device=w.device)
+        ops().rms_act_bwd(xc, w, rstd, dy.contiguous(), None, None, dx, dw, ctx.act)
         return dx, dw.to(ctx.wdtype), None, None, None
 
 
@@ -54,11 +60,11 @@ class _RmsActSkip(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, eps, act, lead):
         xc = x.contiguous()
-        w32 = weight.detach().float().contiguous()
+        w = _weight(weight)
         y = torch.empty_like(xc)
         rstd = torch.empty(xc.numel() // xc.shape[-1], dtype=torch.float32, device=x.device)
-        ops().rms_act_fwd(xc, w32, y, rstd, eps, act)
-        ctx.save_for_backward(xc, w32, rstd)
+        ops().rms_act_fwd(xc, w, y, rstd, eps, act)
+        ctx.save_for_backward(xc, w, rstd)
         ctx.act, ctx.wdtype, ctx.lead = act, weight.dtype, lead
         if lead:
             return y, x.view_as(x), y[..., :lead].contiguous()
@@ -66,13 +72,13 @@ class _RmsActSkip(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy, dskip, dlead=None):
-        xc, w32, rstd = ctx.saved_tensors
+        xc, w, rstd = ctx.saved_tensors
         if dy.dtype not in (torch.bfloat16, torch.float32):
             dy = dy.float()
         dx = torch.empty_like(xc)
-        dw = torch.zeros_like(w32)
+        dw = torch.zeros(w.shape, dtype=torch.float32, device=w.device)
         lead = dlead.to(dy.dtype).contiguous() if (ctx.lead and dlead is not None) else None
-        ops().rms_act_bwd(xc, w32, rstd, dy.contiguous(), dskip.to(xc.dtype).contiguous(), lead, dx, dw, ctx.act)
+        ops().rms_act_bwd(xc, w, rstd, dy.contiguous(), dskip.to(xc.dtype).contiguous(), lead, dx, dw, ctx.act)
         return dx, dw.to(ctx.wdtype), None, None, None
 
 

@@ -135,6 +135,26 @@ def test_rms_norm_act(C, act, dtypes):
     assert _rel(xa.grad, xb.grad) < tol and _rel(wa.grad, wb.grad) < tol
 
 
+@pytest.mark.parametrize("C", [256, 300, 512, 768, 1024, 1280])
+@pytest.mark.parametrize("rows,off", [(1, 0), (37, 0), (6001, 0), (37, 1)])
+def test_rms_norm_act_with_bf16_weights_is_the_same_as_with_their_fp32_values(C, rows, off):
+    """Weights are read in either type; rows on and off the 16-byte boundary (the latter take the general path)."""
+    from ml_experiments_b200.ops.norm_act import rms_norm_act, rms_norm_act_ref
+
+    g = torch.Generator().manual_seed(C + rows)
+    x = torch.randn(rows * C + 8, generator=g).bfloat16().cuda()[off:off + rows * C].view(rows, C)
+    w = (torch.rand(C, generator=g) + 0.5).bfloat16().cuda()
+    xa, wa, xb, wb = x.clone().requires_grad_(), w.clone().requires_grad_(), x.clone().requires_grad_(), w.float().requires_grad_()
+    if off:
+        xa, xb = x.detach().requires_grad_(), x.detach().requires_grad_()
+    ya, yb = rms_norm_act(xa, wa, 1e-6, "silu"), rms_norm_act(xb, wb, 1e-6, "silu")
+    assert torch.equal(ya, yb) and _rel(ya, rms_norm_act_ref(x.float(), w.float(), 1e-6, "silu")) < 4e-3
+    gy = torch.randn(rows, C, generator=g).bfloat16().cuda()
+    ya.backward(gy)
+    yb.backward(gy)
+    assert torch.equal(xa.grad, xb.grad) and wa.grad.dtype == torch.bfloat16 and _rel(wa.grad, wb.grad) < 4e-3
+
+
 @pytest.mark.parametrize("C,dtype,lead", [(768, torch.bfloat16, 12), (1024, torch.bfloat16, 0), (512, torch.bfloat16, 9), (300, torch.bfloat16, 12),
                                           (256, torch.float32, 5)])
 def test_rms_norm_act_skip_adds_the_skip_gradient_in_the_backward_kernel(C, dtype, lead):
