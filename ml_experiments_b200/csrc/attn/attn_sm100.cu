@@ -506,36 +506,34 @@ __global__ void attn_delta_vec_kernel(const __nv_bfloat16* __restrict__ o, long 
 // ------------------------------------------------------------------------------------------------
 // backward
 // ------------------------------------------------------------------------------------------------
-// Warps 0-7 compute (warps w and w+4 share TMEM lane quarter (w & 3) and split the columns of every accumulator in halves),
-// warp 8 issues the MMAs, warp 9 the TMA loads. The tensor pipe runs the products in issue order, per query tile `it`:
+// Head_dim 128. Warps 0-7 compute (warps w and w+4 share TMEM lane quarter (w & 3) and split the columns of S and dP), four warps
+// drain dQ, one issues the MMAs, one the TMA loads. The tensor pipe runs the products in issue order, per query tile `it`:
 //   S, dP of tile it+1   as soon as every warp has copied tile it's S / dP out of TMEM: under the exponentials of tile it;
-//   dQ of tile it        right behind the exponentials, on its own barrier; it is drained after the exponentials of tile
-//                        it+1, so nobody waits for it;
-//   dV, dK of tile it    their barrier is waited for before the P / dS staging is overwritten.
-// At head_dim 128 Pᵀ and dSᵀ are the A operands of dV / dK from tensor memory (dSᵀ is in shared memory too, for dQ); at
-// head_dim 64, with half the shared-memory traffic, staging both there is faster (2.95 ms against 3.28 ms below).
-// Bound: shared memory. At 64 queries a tile S, dP and dQ take 6 KB of operands per 32 cycles of MMA, 48 cycles at
-// 128 bytes a clock; with the operands of dV / dK, the staging and the loads it is about 2100 cycles a tile (D = 128).
-// Measured, 16384 tokens causal: 6 heads of 128 1.29 ms = 796 TFLOP/s (2.05 ms with the MMAs issued by single threads of the
-// compute warps, dQ drained in the tile that formed it and a branch per masked pair), 16 heads of 64 3.01 ms (4.65 ms);
-// 20011 tokens in documents of 700, 16 heads of 64: 0.361 ms (0.505 ms).
-constexpr int BWD_THREADS = 320;
+//   dQ of tile it        right behind the exponentials, on its own barrier, drained by warps that do nothing else;
+//   dV, dK of tile it    their barrier is waited for before P / dS are overwritten.
+// Pᵀ and dSᵀ are the A operands of dV / dK from tensor memory; dSᵀ is in shared memory too, for dQ.
+// Bound: shared memory, 288 KB a tile of 128 keys x 64 queries (S, dP and dQ read 6 KB of operands per MMA, dQ is staged, Q and dO
+// arrive): 2300 cycles at 128 bytes a clock, of 2600. Measured, 16384 tokens causal, 6 heads: 0.965 ms = 1070 TFLOP/s (1.28 ms with dQ
+// drained by the compute warps, whose copy, fence and barrier were 900 cycles a tile with nothing to run under them, and shared
+// memory behind generic addresses); documents of 1024, 49152 tokens: 0.360 ms (0.433 ms). Four warps a lane quarter: 0.98 ms.
+constexpr int BWD_PARTS = 2, BWD_WARPS = 4 * BWD_PARTS, BWD_COMPUTE = 32 * BWD_WARPS, BWD_THREADS = BWD_COMPUTE + 128 + 64;
+constexpr int BWD64_QB = 6;
+constexpr int BWD_MMA = BWD_WARPS + 4, BWD_TMA = BWD_MMA + 1;   // the warps after the four that drain dQ
 
-template <int D>
 __global__ void __launch_bounds__(BWD_THREADS, 1)
-attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
+attn_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
                 const __grid_constant__ CUtensorMap tmdQ, const KP p) {
-  constexpr int NS = D / 64;
+  constexpr int D = 128, NS = D / 64;
   constexpr int BKV = 128, BQ = 64;
   constexpr int KV_BYTES = NS * BKV * 128;  // K or V tile
   constexpr int Q_BYTES = NS * BQ * 128;    // Q or dO tile
-  constexpr bool TS = D == 128;             // Pᵀ and dSᵀ of dV / dK in tensor memory (else in shared memory)
-  constexpr int DS_BYTES = BKV * 128;       // dSᵀ or Pᵀ: 128 key rows x 64 queries
+  constexpr int DS_BYTES = BKV * 128;       // dSᵀ: 128 key rows x 64 queries
   constexpr int DQ_BYTES = BQ * D * 4;      // fp32 staging of one dQ tile
   constexpr uint32_t ST_COL = 0, DPT_COL = 64, DV_COL = 128, DK_COL = 128 + D, DQT_COL = 128 + 2 * D;
   constexpr uint32_t P16_COL = DQT_COL + 64, DS16_COL = P16_COL + 32;   // Pᵀ and dSᵀ as packed bf16: A operands of dV, dK
   constexpr uint32_t TMEM_COLS = 512;
+  static_assert(DS16_COL + 32 <= TMEM_COLS, "tensor memory");
 
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw + (-smem_u32(smem_raw) & 1023u);
@@ -545,8 +543,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint8_t* sQ = sV + KV_BYTES;
   uint8_t* sdO = sQ + NQB * Q_BYTES;
   uint8_t* sdST = sdO + NQB * Q_BYTES;
-  uint8_t* sPT = sdST + DS_BYTES;     // not there with TS
-  float* sdQ = reinterpret_cast<float*>(sPT + (TS ? 0 : DS_BYTES));
+  float* sdQ = reinterpret_cast<float*>(sdST + DS_BYTES);
   float2* s_ld_all = reinterpret_cast<float2*>(reinterpret_cast<uint8_t*>(sdQ) + DQ_BYTES);  // [2][64] {lse, delta}, double-buffered over query tiles
   int* s_ds_all = reinterpret_cast<int*>(s_ld_all + 2 * BQ);      // [2][64] document start of each query
   uint64_t* bars = reinterpret_cast<uint64_t*>(s_ds_all + 2 * BQ);
@@ -567,7 +564,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int lane = tid & 31;
   const int quarter = warp & 3;
-  const int half = (warp >> 2) & 1;
+  const int part = (warp >> 2) & (BWD_PARTS - 1);   // its columns: CQ queries, D / BWD_PARTS of the head dimension
+  constexpr int CQ = BQ / BWD_PARTS, CD = D / BWD_PARTS;
   const int r = quarter * 32 + lane;  // accumulator row owned by this thread
   const int jb = blockIdx.x;
   const int h = blockIdx.y;
@@ -599,14 +597,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     mbar_init(bar_m1, 1);
     mbar_init(bar_m2, 1);
     mbar_init(bar_dq, 1);
-    mbar_init(bar_sfree, 8);
-    mbar_init(bar_pds, 8);
-    mbar_init(bar_dqfree, 8);
+    mbar_init(bar_sfree, BWD_WARPS);
+    mbar_init(bar_pds, BWD_WARPS);
+    mbar_init(bar_dqfree, 4);
     for (int i = 0; i < NQB; ++i) { mbar_init(&bar_q[i], 1); mbar_init(&bar_qe[i], 1); }
     *abort_flag = 0;
     fence_mbar_init();
   }
-  if (warp == 8) {
+  if (warp == BWD_MMA) {
     tmem_alloc(tmem_slot, TMEM_COLS);
     tmem_relinquish();
   }
@@ -615,12 +613,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
   if (leave) {
-    if (warp == 8) tmem_dealloc(tmem_base, TMEM_COLS);
+    if (warp == BWD_MMA) tmem_dealloc(tmem_base, TMEM_COLS);
     return;
   }
   const uint32_t lane_off = uint32_t(quarter * 32) << 16;
 
-  if (warp == 9) {
+  if (warp == BWD_TMA) {
     if (elect_one_sync()) {
       mbar_arrive_expect_tx(bar_kv, 2 * KV_BYTES);
       for (int s = 0; s < NS; ++s) {
@@ -638,7 +636,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         }
       }
     }
-  } else if (warp == 8) {
+  } else if (warp == BWD_MMA) {
     // the whole warp walks the tiles and one elected lane issues: operands stay in uniform registers (see the forward)
     const uint32_t idesc_st = make_idesc(FMT_BF16, FMT_BF16, 0, 0, 128, BQ);   // K·Qᵀ, V·dOᵀ
     const uint32_t idesc_dv = make_idesc(FMT_BF16, FMT_BF16, 0, 1, 128, D);    // Pᵀ·dO, dSᵀ·Q   (B MN-major)
@@ -647,7 +645,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const uint64_t kd = make_smem_desc_sw128(smem_u32(sK), 16, 1024), vd = make_smem_desc_sw128(smem_u32(sV), 16, 1024);
     const uint64_t qd = make_smem_desc_sw128(smem_u32(sQ), 16, 1024), dod = make_smem_desc_sw128(smem_u32(sdO), 16, 1024);
     const uint64_t kmn = make_smem_desc_sw128(smem_u32(sK), BKV * 128, 1024), dsmn = make_smem_desc_sw128(smem_u32(sdST), BKV * 128, 1024);
-    const uint64_t ptd = make_smem_desc_sw128(smem_u32(sPT), 16, 1024), dsd = make_smem_desc_sw128(smem_u32(sdST), 16, 1024);
     const uint64_t qmn = make_smem_desc_sw128(smem_u32(sQ), BQ * 128, 1024), domn = make_smem_desc_sw128(smem_u32(sdO), BQ * 128, 1024);
     auto issue_s_dp = [&](int it) {
       const int buf = it % NQB;
@@ -656,13 +653,15 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const uint64_t off = buf * (Q_BYTES / 16);
       if (elect_one_sync()) {
 #pragma unroll
-        for (int ks = 0; ks < D / 16; ++ks)
-          tc_mma_f16(tmem_base + ST_COL, kd + ((ks / 4) * (BKV * 128) + (ks % 4) * 32) / 16,
-                     qd + off + ((ks / 4) * (BQ * 128) + (ks % 4) * 32) / 16, idesc_st, ks != 0);
+        for (int ks = 0; ks < D / 16; ++ks) {
+          const uint64_t bd = qd + off + ((ks / 4) * (BQ * 128) + (ks % 4) * 32) / 16;
+          tc_mma_f16(tmem_base + ST_COL, kd + ((ks / 4) * (BKV * 128) + (ks % 4) * 32) / 16, bd, idesc_st, ks != 0);
+        }
 #pragma unroll
-        for (int ks = 0; ks < D / 16; ++ks)
-          tc_mma_f16(tmem_base + DPT_COL, vd + ((ks / 4) * (BKV * 128) + (ks % 4) * 32) / 16,
-                     dod + off + ((ks / 4) * (BQ * 128) + (ks % 4) * 32) / 16, idesc_st, ks != 0);
+        for (int ks = 0; ks < D / 16; ++ks) {
+          const uint64_t bd = dod + off + ((ks / 4) * (BQ * 128) + (ks % 4) * 32) / 16;
+          tc_mma_f16(tmem_base + DPT_COL, vd + ((ks / 4) * (BKV * 128) + (ks % 4) * 32) / 16, bd, idesc_st, ks != 0);
+        }
         tc_commit(bar_m1);
       }
       __syncwarp();
@@ -690,50 +689,57 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 #pragma unroll
         for (int ks = 0; ks < BQ / 16; ++ks) { // dV += Pᵀ · dO
           const uint64_t bd = domn + off + ks * (2048 / 16);
-          if constexpr (TS) tc_mma_f16_ts(tmem_base + DV_COL, tmem_base + P16_COL + ks * 8, bd, idesc_dv, (it | ks) != 0);
-          else tc_mma_f16(tmem_base + DV_COL, ptd + ks * (32 / 16), bd, idesc_dv, (it | ks) != 0);
+          tc_mma_f16_ts(tmem_base + DV_COL, tmem_base + P16_COL + ks * 8, bd, idesc_dv, (it | ks) != 0);
         }
 #pragma unroll
         for (int ks = 0; ks < BQ / 16; ++ks) { // dK += dSᵀ · Q
           const uint64_t bd = qmn + off + ks * (2048 / 16);
-          if constexpr (TS) tc_mma_f16_ts(tmem_base + DK_COL, tmem_base + DS16_COL + ks * 8, bd, idesc_dv, (it | ks) != 0);
-          else tc_mma_f16(tmem_base + DK_COL, dsd + ks * (32 / 16), bd, idesc_dv, (it | ks) != 0);
+          tc_mma_f16_ts(tmem_base + DK_COL, tmem_base + DS16_COL + ks * 8, bd, idesc_dv, (it | ks) != 0);
         }
         tc_commit(&bar_qe[buf]);
         tc_commit(bar_m2);        // the last one is waited for: no report may come after the CTA has ended
       }
       __syncwarp();
     }
+  } else if (warp >= BWD_WARPS) {
+    // dQᵀ of a tile (row = head-dim index r) -> staging[q][r], then one bulk reduce-add into the fp32 accumulator (reductions
+    // issued element by element from registers measured 25 % slower). Warps of their own: in the compute warps this copy, its
+    // fence and its barrier were 900 of 2850 cycles a tile, with nothing to run under them.
+    const bool issue_red = tid == BWD_COMPUTE;
+    auto drain_sync = [] { asm volatile("bar.sync 2, 128;" ::: "memory"); };
+    for (int it = 0; it < ntile; ++it) {
+      cta_wait(bar_dq, it & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL);
+      tc_fence_after_sync();
+      uint32_t v[2][32];
+      if (r < D) {
+        tmem_ld_32x32b_x32(tmem_base + lane_off + DQT_COL, v[0]);
+        tmem_ld_32x32b_x32(tmem_base + lane_off + DQT_COL + 32, v[1]);
+        tmem_ld_wait();
+      }
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_dqfree);
+      if (issue_red) tma_store_wait_read<0>();   // the last reduce-add has drained the staging buffer
+      drain_sync();
+      if (r < D) {
+#pragma unroll
+        for (int i = 0; i < BQ; ++i) sdQ[i * D + r] = __uint_as_float(v[i / 32][i % 32]) * p.scale;
+      }
+      fence_proxy_async_smem();
+      drain_sync();                              // the staged tile is complete
+      if (issue_red) {
+        tma_reduce_add_3d(&tmdQ, sdQ, 0, q_lo + it * BQ, h);
+        tma_store_commit();
+      }
+    }
+    if (issue_red) tma_store_wait_read<0>();     // shared memory may be given back
   } else {
-    const bool issue_red = tid == 64;
-    auto compute_sync = [] { asm volatile("bar.sync 1, 256;" ::: "memory"); };
+    auto compute_sync = [] { asm volatile("bar.sync 1, %0;" ::"n"(BWD_COMPUTE) : "memory"); };
     if (tid < BQ) {
       s_ld_all[tid] = nxt_ld;
       s_ds_all[tid] = nxt_ds;
     }
     compute_sync();
-    // dQᵀ row (= head-dim index r) of tile it, this warp's half of the query columns -> staging[q][r], then one bulk
-    // reduce-add into the fp32 accumulator (reductions issued element by element from registers measured 25 % slower)
-    auto drain_dq = [&](int it) {
-      cta_wait(bar_dq, it & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL);
-      tc_fence_after_sync();
-      uint32_t v[32];
-      tmem_ld_32x32b_x32(tmem_base + lane_off + DQT_COL + half * 32, v);
-      tmem_ld_wait();
-      tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar_dqfree);
-      if (r < D) {      // the staging buffer is free: see the barrier in front of the call
-#pragma unroll
-        for (int i = 0; i < 32; ++i) sdQ[(half * 32 + i) * D + r] = __uint_as_float(v[i]) * p.scale;
-      }
-      fence_proxy_async_smem();
-      compute_sync();                            // the staged tile is complete
-      if (issue_red) {
-        tma_reduce_add_3d(&tmdQ, sdQ, 0, q_lo + it * BQ, h);
-        tma_store_commit();
-      }
-    };
     for (int it = 0; it < ntile; ++it) {
       const int qt0 = q_lo + it * BQ;
       const float2* s_ld = s_ld_all + (it & 1) * BQ;
@@ -742,9 +748,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       if (it + 2 < ntile) scalars(qt0 + 2 * BQ, far_ld, far_ds);
       cta_wait(bar_m1, it & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL);
       tc_fence_after_sync();
-      uint32_t sv[32], dv_[32];
-      tmem_ld_32x32b_x32(tmem_base + lane_off + ST_COL + half * 32, sv);
-      tmem_ld_32x32b_x32(tmem_base + lane_off + DPT_COL + half * 32, dv_);
+      uint32_t sv[CQ], dv_[CQ];
+      tmem_ld_32x32b_x32(tmem_base + lane_off + ST_COL + part * CQ, sv);
+      tmem_ld_32x32b_x32(tmem_base + lane_off + DPT_COL + part * CQ, dv_);
       tmem_ld_wait();
       tc_fence_before_sync();
       __syncwarp();
@@ -754,32 +760,32 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const bool need_mask = (qt0 < kv0 + BKV) || (s_ds[BQ - 1] > kv0) || (kv0 + BKV > p.T) || (qt0 + BQ > p.T);
       // probabilities, then the mask in a loop of its own: a branch per element would serialise the latencies of the others
 #pragma unroll
-      for (int i = 0; i < 32; i += 2) {
-        const float4 ld = *reinterpret_cast<const float4*>(&s_ld[half * 32 + i]);   // {lse, delta} of two queries
+      for (int i = 0; i < CQ; i += 2) {
+        const float4 ld = *reinterpret_cast<const float4*>(&s_ld[part * CQ + i]);   // {lse, delta} of two queries
         sv[i] = __float_as_uint(exp2f(fmaf(__uint_as_float(sv[i]), p.sl2, -ld.x)));
         sv[i + 1] = __float_as_uint(exp2f(fmaf(__uint_as_float(sv[i + 1]), p.sl2, -ld.z)));
         dv_[i] = __float_as_uint(__uint_as_float(dv_[i]) - ld.y);
         dv_[i + 1] = __float_as_uint(__uint_as_float(dv_[i + 1]) - ld.w);
       }
       if (need_mask) {
-        // queries [lo, hi) of this thread's 32 see its key: from the key itself to the last query whose document has begun at
+        // queries [lo, hi) of this thread's see its key: from the key itself to the last query whose document has begun at
         // or before it (document starts never fall, so that is a search for the first later one)
-        const int lo = kv - qt0 - half * 32;
-        int hi = 32;
-        if (s_ds[half * 32 + 31] > kv) {
+        const int lo = kv - qt0 - part * CQ;
+        int hi = CQ;
+        if (s_ds[part * CQ + CQ - 1] > kv) {
           hi = 0;
 #pragma unroll
-          for (int step = 16; step > 0; step >>= 1)
-            if (s_ds[half * 32 + hi + step - 1] <= kv) hi += step;
+          for (int step = CQ / 2; step > 0; step >>= 1)
+            if (s_ds[part * CQ + hi + step - 1] <= kv) hi += step;
         }
         if (kv >= p.T) hi = 0;
 #pragma unroll
-        for (int i = 0; i < 32; ++i)
+        for (int i = 0; i < CQ; ++i)
           if (i < lo || i >= hi) sv[i] = 0u;
       }
-      uint32_t pp[16], dd[16];
+      uint32_t pp[CQ / 2], dd[CQ / 2];
 #pragma unroll
-      for (int i = 0; i < 32; i += 2) {
+      for (int i = 0; i < CQ; i += 2) {
         const float p0 = __uint_as_float(sv[i]), p1 = __uint_as_float(sv[i + 1]);
         pp[i >> 1] = pack_bf16x2(p0, p1);
         dd[i >> 1] = pack_bf16x2(p0 * __uint_as_float(dv_[i]), p1 * __uint_as_float(dv_[i + 1]));
@@ -788,80 +794,57 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         s_ld_all[((it + 1) & 1) * BQ + tid] = nxt_ld;
         s_ds_all[((it + 1) & 1) * BQ + tid] = nxt_ds;
       }
-      if (issue_red) tma_store_wait_read<0>();   // the last reduce-add has drained the dQ staging buffer
-      compute_sync();                            // ... and the next tile's scalars are visible
+      compute_sync();                            // the next tile's scalars are visible
       if (it > 0) {
-        drain_dq(it - 1);
         cta_wait(bar_m2, (it - 1) & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL);   // P / dS of the last tile are free
         tc_fence_after_sync();
       }
-      if constexpr (TS) {
-        tmem_st_32x32b_x16(tmem_base + lane_off + P16_COL + half * 16, pp);
-        tmem_st_32x32b_x16(tmem_base + lane_off + DS16_COL + half * 16, dd);
-      }
+      tmem_st_32x32b_x16(tmem_base + lane_off + P16_COL + part * (CQ / 2), pp);
+      tmem_st_32x32b_x16(tmem_base + lane_off + DS16_COL + part * (CQ / 2), dd);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int at = r * 128 + (((half * 4 + j) ^ (r & 7)) << 4);
-        if constexpr (!TS) *reinterpret_cast<uint4*>(sPT + at) = make_uint4(pp[4 * j], pp[4 * j + 1], pp[4 * j + 2], pp[4 * j + 3]);
+      for (int j = 0; j < CQ / 8; ++j) {
+        const int at = r * 128 + (((part * (CQ / 8) + j) ^ (r & 7)) << 4);
         *reinterpret_cast<uint4*>(sdST + at) = make_uint4(dd[4 * j], dd[4 * j + 1], dd[4 * j + 2], dd[4 * j + 3]);
       }
-      if constexpr (TS) tmem_st_wait();
+      tmem_st_wait();
       fence_proxy_async_smem();
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_pds);
     }
-    if (ntile > 0) {
-      if (issue_red) tma_store_wait_read<0>();
-      compute_sync();
-      drain_dq(ntile - 1);
-    }
-
-    // final: dV, dK rows; each warp writes its half of the head dimension
+    // final: dV, dK rows; each warp writes its part of the head dimension
     if (ntile > 0) cta_wait(bar_m2, (ntile - 1) & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL);
     tc_fence_after_sync();
+    __nv_bfloat16* dvrow = p.dv + (long long)kv * p.ld_dv + h * D + part * CD;
+    __nv_bfloat16* dkrow = p.dk + (long long)kv * p.ld_dk + h * D + part * CD;
     if (ntile > 0) {
-      __nv_bfloat16* dvrow = p.dv + (long long)kv * p.ld_dv + h * D + half * (D / 2);
-      __nv_bfloat16* dkrow = p.dk + (long long)kv * p.ld_dk + h * D + half * (D / 2);
+      auto write = [&](uint32_t col, __nv_bfloat16* row, float mul) {
 #pragma unroll
-      for (int c = 0; c < D / 64; ++c) {
-        uint32_t v[32];
-        tmem_ld_32x32b_x32(tmem_base + lane_off + DV_COL + half * (D / 2) + c * 32, v);
-        tmem_ld_wait();
-        if (kv < p.T) {
+        for (int c = 0; c < CD; c += 16) {
+          uint32_t v[16];
+          tmem_ld_32x32b_x16(tmem_base + lane_off + col + part * CD + c, v);
+          tmem_ld_wait();
+          if (kv < p.T) {
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            uint4 u = make_uint4(pack_bf16x2(__uint_as_float(v[8 * j]), __uint_as_float(v[8 * j + 1])),
-                                 pack_bf16x2(__uint_as_float(v[8 * j + 2]), __uint_as_float(v[8 * j + 3])),
-                                 pack_bf16x2(__uint_as_float(v[8 * j + 4]), __uint_as_float(v[8 * j + 5])),
-                                 pack_bf16x2(__uint_as_float(v[8 * j + 6]), __uint_as_float(v[8 * j + 7])));
-            reinterpret_cast<uint4*>(dvrow + c * 32)[j] = u;
+            for (int j = 0; j < 2; ++j)
+              reinterpret_cast<uint4*>(row + c)[j] =
+                  make_uint4(pack_bf16x2(__uint_as_float(v[8 * j]) * mul, __uint_as_float(v[8 * j + 1]) * mul),
+                             pack_bf16x2(__uint_as_float(v[8 * j + 2]) * mul, __uint_as_float(v[8 * j + 3]) * mul),
+                             pack_bf16x2(__uint_as_float(v[8 * j + 4]) * mul, __uint_as_float(v[8 * j + 5]) * mul),
+                             pack_bf16x2(__uint_as_float(v[8 * j + 6]) * mul, __uint_as_float(v[8 * j + 7]) * mul));
           }
         }
-        tmem_ld_32x32b_x32(tmem_base + lane_off + DK_COL + half * (D / 2) + c * 32, v);
-        tmem_ld_wait();
-        if (kv < p.T) {
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            uint4 u = make_uint4(pack_bf16x2(__uint_as_float(v[8 * j]) * p.scale, __uint_as_float(v[8 * j + 1]) * p.scale),
-                                 pack_bf16x2(__uint_as_float(v[8 * j + 2]) * p.scale, __uint_as_float(v[8 * j + 3]) * p.scale),
-                                 pack_bf16x2(__uint_as_float(v[8 * j + 4]) * p.scale, __uint_as_float(v[8 * j + 5]) * p.scale),
-                                 pack_bf16x2(__uint_as_float(v[8 * j + 6]) * p.scale, __uint_as_float(v[8 * j + 7]) * p.scale));
-            reinterpret_cast<uint4*>(dkrow + c * 32)[j] = u;
-          }
-        }
-      }
+      };
+      write(DV_COL, dvrow, 1.f);
+      write(DK_COL, dkrow, p.scale);
     } else if (kv < p.T) {
       // no query tile attends this key tile: its gradients are zero (the caller does not pre-zero dk / dv)
-      __nv_bfloat16* dvrow = p.dv + (long long)kv * p.ld_dv + h * D + half * (D / 2);
-      __nv_bfloat16* dkrow = p.dk + (long long)kv * p.ld_dk + h * D + half * (D / 2);
 #pragma unroll
-      for (int j = 0; j < D / 16; ++j) {
+      for (int j = 0; j < CD / 8; ++j) {
         reinterpret_cast<uint4*>(dvrow)[j] = make_uint4(0u, 0u, 0u, 0u);
         reinterpret_cast<uint4*>(dkrow)[j] = make_uint4(0u, 0u, 0u, 0u);
       }
     }
-    if (issue_red) tma_store_wait_all<0>();
   }
   __syncwarp();
   if (tid == 0) {
@@ -873,7 +856,347 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  if (warp == 8) tmem_dealloc(tmem_base, TMEM_COLS);
+  if (warp == BWD_MMA) tmem_dealloc(tmem_base, TMEM_COLS);
+}
+
+// Head_dim 64. Two groups of four compute warps take the query tiles in turn (warp w of a group: TMEM lane quarter w & 3, thread = key),
+// four warps drain dQ, one issues the MMAs, one the TMA loads. Tensor memory holds three buffers of 128 columns, tile it in buffer
+// it % 3: its S | dP, then Pᵀ | dSᵀ as packed bf16 (A operands of dV, dK) over S and dQᵀ over dP; a buffer is free again when
+// the tile's products are done (they run in issue order) and its dQᵀ has been copied. So the scores of a group's next tile are
+// ready when it has finished one, and it waits for nothing else. dSᵀ is in shared memory too, for dQ.
+// The tensor pipe runs, per query tile `it`: S, dP of tile it+2; then, behind the group that has tile it, dQ, dV and dK of tile it.
+// Measured, 16384 tokens causal, 16 heads: 1.76 ms = 780 TFLOP/s (3.00 ms with all eight warps on one tile and its scores behind
+// the copy of its own; 2.00 with two buffers; 2.13 with one group and K and V, as A operands, in tensor memory); documents of about
+// 5000: 0.67 ms (1.07), of 700, 20011 tokens: 0.28 ms (0.39). A group needs some 2100 cycles a tile (64 exponentials a thread, one warp
+// a scheduler), two tiles at a time.
+__global__ void __launch_bounds__(BWD_THREADS, 1)
+attn_bwd64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
+                const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
+                const __grid_constant__ CUtensorMap tmdQ, const KP p) {
+  constexpr int D = 64;
+  constexpr int BKV = 128, BQ = 64;
+  constexpr int KV_BYTES = BKV * 128;       // K or V tile
+  constexpr int Q_BYTES = BQ * 128;         // Q or dO tile
+  constexpr int DS_BYTES = BKV * 128;       // dSᵀ: 128 key rows x 64 queries, one for each buffer
+  constexpr int DQ_BYTES = BQ * D * 4;      // fp32 staging of one dQ tile
+  constexpr int NB = 3;                     // buffers in tensor memory, and of dSᵀ
+  constexpr uint32_t BUF = 128, DP_COL = 64, P16_COL = 0, DS16_COL = 32, DQT_COL = 64;     // in a buffer
+  constexpr uint32_t DV_COL = NB * BUF, DK_COL = DV_COL + D;
+  constexpr uint32_t TMEM_COLS = 512;
+  static_assert(DK_COL + D <= TMEM_COLS, "tensor memory");
+
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = smem_raw + (-smem_u32(smem_raw) & 1023u);
+  uint8_t* sK = smem;
+  uint8_t* sV = sK + KV_BYTES;
+  constexpr int NQB = BWD64_QB;       // Q / dO buffers: tiles it to it+2 are in use, the others on their way
+  uint8_t* sQ = sV + KV_BYTES;
+  uint8_t* sdO = sQ + NQB * Q_BYTES;
+  uint8_t* sdST = sdO + NQB * Q_BYTES;
+  float* sdQ = reinterpret_cast<float*>(sdST + NB * DS_BYTES);
+  float2* s_ld_all = reinterpret_cast<float2*>(reinterpret_cast<uint8_t*>(sdQ) + DQ_BYTES);  // [group][2][64] {lse, delta}, for its tiles in turn
+  int* s_ds_all = reinterpret_cast<int*>(s_ld_all + 4 * BQ);      // [group][2][64] document start of each query
+  uint64_t* bars = reinterpret_cast<uint64_t*>(s_ds_all + 4 * BQ);
+  uint64_t* bar_m1 = bars;              // [NB] S / dP of a tile are in TMEM
+  uint64_t* bar_pds = bars + NB;        // [NB] P / dS of a tile are in place, one arrival per warp of the group
+  uint64_t* bar_dq = bars + 2 * NB;     // [NB] dQ of a tile is in TMEM
+  uint64_t* bar_dqfree = bars + 3 * NB; // [NB] and in registers, one arrival per drain warp
+  uint64_t* bar_q = bars + 4 * NB;      // [NQB] a Q / dO buffer is full
+  uint64_t* bar_qe = bar_q + NQB;       // [NQB] and empty again
+  uint64_t* bar_kv = bar_qe + NQB;
+  uint64_t* bar_done = bar_kv + 1;      // dV and dK are complete
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_done + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const bool poisoned = status_poisoned(p.status);
+  const int tid = threadIdx.x;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  const int lane = tid & 31;
+  const int quarter = warp & 3;
+  const int group = (warp >> 2) & 1;
+  const int r = quarter * 32 + lane;  // accumulator row of this thread
+  const int jb = blockIdx.x;
+  const int h = blockIdx.y;
+  const int kv0 = jb * BKV;
+  const int kv = kv0 + r;
+
+  // query range that can see any key of this tile
+  const int last_kv = min(kv0 + BKV, p.T) - 1;
+  int q_hi = p.doc_end[last_kv];
+  if (p.window_blocks > 0) q_hi = min(q_hi, (jb + p.window_blocks) * 128);
+  q_hi = min(q_hi, p.T);
+  const int q_lo = kv0;
+  const int ntile = (q_hi - q_lo + BQ - 1) / BQ;
+  // per-query scalars (lse, delta, document start) of a group's next tile are loaded while it works on a tile; those of the first are
+  // on their way during the set-up
+  float2 nxt_ld;
+  int nxt_ds;
+  auto scalars = [&](int it) {
+    const int qq = q_lo + it * BQ + r;
+    const bool okq = r < BQ && it < ntile && qq < p.T;
+    nxt_ld = make_float2(okq ? p.lse[(long long)h * p.T + qq] : INFINITY, okq ? p.delta[(long long)h * p.T + qq] : 0.f);
+    nxt_ds = okq ? p.doc_start[qq] : 0x7fffffff;
+  };
+  scalars(group);
+
+  if (tid == 0) {
+    for (int i = 0; i < NB; ++i) {
+      mbar_init(&bar_m1[i], 1);
+      mbar_init(&bar_pds[i], 4);
+      mbar_init(&bar_dq[i], 1);
+      mbar_init(&bar_dqfree[i], 4);
+    }
+    for (int i = 0; i < NQB; ++i) { mbar_init(&bar_q[i], 1); mbar_init(&bar_qe[i], 1); }
+    mbar_init(bar_kv, 1);
+    mbar_init(bar_done, 1);
+    *abort_flag = 0;
+    fence_mbar_init();
+  }
+  if (warp == BWD_MMA) {
+    tmem_alloc(tmem_slot, TMEM_COLS);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  const bool leave = __syncthreads_or(poisoned);     // all warps or none
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+  if (leave) {
+    if (warp == BWD_MMA) tmem_dealloc(tmem_base, TMEM_COLS);
+    return;
+  }
+  const uint32_t lane_off = uint32_t(quarter * 32) << 16;
+
+  if (warp == BWD_TMA) {
+    if (elect_one_sync()) {
+      mbar_arrive_expect_tx(bar_kv, 2 * KV_BYTES);
+      tma_load_3d(sK, &tmK, bar_kv, 0, kv0, h);
+      tma_load_3d(sV, &tmV, bar_kv, 0, kv0, h);
+      for (int it = 0; it < ntile; ++it) {
+        const int buf = it % NQB;
+        if (it >= NQB) cta_wait(&bar_qe[buf], (it / NQB - 1) & 1, abort_flag, p.status, ERR_WAIT_SMEM_EMPTY);
+        if (*abort_flag) break;
+        mbar_arrive_expect_tx(&bar_q[buf], 2 * Q_BYTES);
+        tma_load_3d(sQ + buf * Q_BYTES, &tmQ, &bar_q[buf], 0, q_lo + it * BQ, h);
+        tma_load_3d(sdO + buf * Q_BYTES, &tmdO, &bar_q[buf], 0, q_lo + it * BQ, h);
+      }
+    }
+  } else if (warp == BWD_MMA) {
+    // the whole warp walks the tiles and one elected lane issues: operands stay in uniform registers (see the forward)
+    const uint32_t idesc_st = make_idesc(FMT_BF16, FMT_BF16, 0, 0, 128, BQ);   // K·Qᵀ, V·dOᵀ
+    const uint32_t idesc_dv = make_idesc(FMT_BF16, FMT_BF16, 0, 1, 128, D);    // Pᵀ·dO, dSᵀ·Q   (B MN-major)
+    const uint32_t idesc_dq = make_idesc(FMT_BF16, FMT_BF16, 1, 1, 128, BQ);   // Kᵀ·dSᵀ         (A, B MN-major)
+    // descriptors differ in their start address only (its unit is 16 bytes)
+    const uint64_t kd = make_smem_desc_sw128(smem_u32(sK), 16, 1024), vd = make_smem_desc_sw128(smem_u32(sV), 16, 1024);
+    const uint64_t qd = make_smem_desc_sw128(smem_u32(sQ), 16, 1024), dod = make_smem_desc_sw128(smem_u32(sdO), 16, 1024);
+    const uint64_t kmn = make_smem_desc_sw128(smem_u32(sK), BKV * 128, 1024), dsmn = make_smem_desc_sw128(smem_u32(sdST), BKV * 128, 1024);
+    const uint64_t qmn = make_smem_desc_sw128(smem_u32(sQ), BQ * 128, 1024), domn = make_smem_desc_sw128(smem_u32(sdO), BQ * 128, 1024);
+    auto issue_s_dp = [&](int it) {
+      const int buf = it % NQB, b = it % NB;
+      cta_wait(&bar_q[buf], (it / NQB) & 1, abort_flag, p.status, ERR_WAIT_SMEM_FULL);
+      if (it >= NB) cta_wait(&bar_dqfree[b], (it / NB - 1) & 1, abort_flag, p.status, ERR_WAIT_TMEM_EMPTY);
+      tc_fence_after_sync();
+      const uint64_t off = buf * (Q_BYTES / 16);
+      const uint32_t s_col = tmem_base + b * BUF;
+      if (elect_one_sync()) {
+#pragma unroll
+        for (int ks = 0; ks < D / 16; ++ks) tc_mma_f16(s_col, kd + ks * 2, qd + off + ks * 2, idesc_st, ks != 0);
+#pragma unroll
+        for (int ks = 0; ks < D / 16; ++ks) tc_mma_f16(s_col + DP_COL, vd + ks * 2, dod + off + ks * 2, idesc_st, ks != 0);
+        tc_commit(&bar_m1[b]);
+      }
+      __syncwarp();
+    };
+    cta_wait(bar_kv, 0, abort_flag, p.status, ERR_WAIT_SMEM_FULL);     // also when no query tile reads them
+    tc_fence_after_sync();
+    if (ntile > 0) issue_s_dp(0);
+    if (ntile > 1) issue_s_dp(1);
+    for (int it = 0; it < ntile; ++it) {
+      if (__any_sync(0xffffffffu, *abort_flag)) break;
+      const int buf = it % NQB, b = it % NB;
+      if (it + 2 < ntile) issue_s_dp(it + 2);
+      cta_wait(&bar_pds[b], (it / NB) & 1, abort_flag, p.status, ERR_WAIT_MISC);
+      tc_fence_after_sync();
+      const uint64_t off = buf * (Q_BYTES / 16), ds = dsmn + b * (DS_BYTES / 16);
+      const uint32_t base = tmem_base + b * BUF;
+      if (elect_one_sync()) {
+#pragma unroll
+        for (int ks = 0; ks < BKV / 16; ++ks)  // dQᵀ = Kᵀ · dSᵀ
+          tc_mma_f16(base + DQT_COL, kmn + ks * (2048 / 16), ds + ks * (2048 / 16), idesc_dq, ks != 0);
+        tc_commit(&bar_dq[b]);
+#pragma unroll
+        for (int ks = 0; ks < BQ / 16; ++ks)   // dV += Pᵀ · dO
+          tc_mma_f16_ts(tmem_base + DV_COL, base + P16_COL + ks * 8, domn + off + ks * (2048 / 16), idesc_dv, (it | ks) != 0);
+#pragma unroll
+        for (int ks = 0; ks < BQ / 16; ++ks)   // dK += dSᵀ · Q
+          tc_mma_f16_ts(tmem_base + DK_COL, base + DS16_COL + ks * 8, qmn + off + ks * (2048 / 16), idesc_dv, (it | ks) != 0);
+        // only what somebody waits for is reported: nothing may come after the CTA has ended
+        if (it + NQB < ntile) tc_commit(&bar_qe[buf]);
+        if (it + 1 == ntile) tc_commit(bar_done);
+      }
+      __syncwarp();
+    }
+  } else if (warp >= BWD_WARPS) {
+    // dQᵀ of a tile (row = head-dim index r) -> staging[q][r], then one bulk reduce-add into the fp32 accumulator (reductions
+    // issued element by element from registers measured 25 % slower). Warps of their own: in the compute warps this copy, its
+    // fence and its barrier were 900 of 2850 cycles a tile, with nothing to run under them.
+    const bool issue_red = tid == BWD_COMPUTE;
+    auto drain_sync = [] { asm volatile("bar.sync 3, 128;" ::: "memory"); };
+    for (int it = 0; it < ntile; ++it) {
+      const int b = it % NB;
+      cta_wait(&bar_dq[b], (it / NB) & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL);
+      tc_fence_after_sync();
+      uint32_t v[2][32];
+      if (r < D) {
+        tmem_ld_32x32b_x32(tmem_base + lane_off + b * BUF + DQT_COL, v[0]);
+        tmem_ld_32x32b_x32(tmem_base + lane_off + b * BUF + DQT_COL + 32, v[1]);
+        tmem_ld_wait();
+      }
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bar_dqfree[b]);
+      if (issue_red) tma_store_wait_read<0>();   // the last reduce-add has drained the staging buffer
+      drain_sync();
+      if (r < D) {
+#pragma unroll
+        for (int i = 0; i < BQ; ++i) sdQ[i * D + r] = __uint_as_float(v[i / 32][i % 32]) * p.scale;
+      }
+      fence_proxy_async_smem();
+      drain_sync();                              // the staged tile is complete
+      if (issue_red) {
+        tma_reduce_add_3d(&tmdQ, sdQ, 0, q_lo + it * BQ, h);
+        tma_store_commit();
+      }
+    }
+    if (issue_red) tma_store_wait_read<0>();     // shared memory may be given back
+  } else {
+    auto group_sync = [&] { asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory"); };
+    for (int it = group; it < ntile; it += 2) {
+      const int qt0 = q_lo + it * BQ, b = it % NB;
+      float2* s_ld = s_ld_all + (it & 3) * BQ;     // (a slower warp may still read those of the group's last tile)
+      int* s_ds = s_ds_all + (it & 3) * BQ;
+      const uint32_t base = tmem_base + lane_off + b * BUF;
+      uint8_t* ds_row = sdST + b * DS_BYTES + r * 128;
+      if (r < BQ) {
+        s_ld[r] = nxt_ld;
+        s_ds[r] = nxt_ds;
+      }
+      group_sync();
+      scalars(it + 2);
+      cta_wait(&bar_m1[b], (it / NB) & 1, abort_flag, p.status, ERR_WAIT_TMEM_FULL);
+      tc_fence_after_sync();
+      uint32_t sv[64], dp[32];
+      {
+        uint32_t a[32], c[32];
+        tmem_ld_32x32b_x32(base, a);
+        tmem_ld_32x32b_x32(base + 32, c);
+        tmem_ld_32x32b_x32(base + DP_COL, dp);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 32; ++i) sv[i] = a[i], sv[32 + i] = c[i];
+      }
+      // masks are needed only where the tile touches the causal diagonal, a document boundary or the sequence end
+      const bool need_mask = (qt0 < kv0 + BKV) || (s_ds[BQ - 1] > kv0) || (kv0 + BKV > p.T) || (qt0 + BQ > p.T);
+      // probabilities, then the mask in a loop of its own: a branch per element would serialise the latencies of the others
+#pragma unroll
+      for (int i = 0; i < 64; i += 2) {
+        const float4 ld = *reinterpret_cast<const float4*>(&s_ld[i]);   // {lse, delta} of two queries
+        sv[i] = __float_as_uint(exp2f(fmaf(__uint_as_float(sv[i]), p.sl2, -ld.x)));
+        sv[i + 1] = __float_as_uint(exp2f(fmaf(__uint_as_float(sv[i + 1]), p.sl2, -ld.z)));
+      }
+      if (need_mask) {
+        // queries [lo, hi) see this thread's key: from the key itself to the last query whose document has begun at
+        // or before it (document starts never fall, so that is a search for the first later one)
+        const int lo = kv - qt0;
+        int hi = 64;
+        if (s_ds[63] > kv) {
+          hi = 0;
+#pragma unroll
+          for (int step = 32; step > 0; step >>= 1)
+            if (s_ds[hi + step - 1] <= kv) hi += step;
+        }
+        if (kv >= p.T) hi = 0;
+#pragma unroll
+        for (int i = 0; i < 64; ++i)
+          if (i < lo || i >= hi) sv[i] = 0u;
+      }
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {          // over S, which this thread, the only reader of its row, has read as a whole
+        uint32_t pp[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) pp[i] = pack_bf16x2(__uint_as_float(sv[32 * c + 2 * i]), __uint_as_float(sv[32 * c + 2 * i + 1]));
+        tmem_st_32x32b_x16(base + P16_COL + c * 16, pp);
+      }
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        if (c == 1) {
+          tmem_ld_32x32b_x32(base + DP_COL + 32, dp);
+          tmem_ld_wait();
+        }
+        uint32_t dd[16];
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) {
+          const float4 ld = *reinterpret_cast<const float4*>(&s_ld[32 * c + i]);
+          dd[i >> 1] = pack_bf16x2(__uint_as_float(sv[32 * c + i]) * (__uint_as_float(dp[i]) - ld.y),
+                                   __uint_as_float(sv[32 * c + i + 1]) * (__uint_as_float(dp[i + 1]) - ld.w));
+        }
+        tmem_st_32x32b_x16(base + DS16_COL + c * 16, dd);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          *reinterpret_cast<uint4*>(ds_row + (((c * 4 + j) ^ (r & 7)) << 4)) = make_uint4(dd[4 * j], dd[4 * j + 1], dd[4 * j + 2], dd[4 * j + 3]);
+      }
+      tmem_st_wait();
+      fence_proxy_async_smem();
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bar_pds[b]);
+    }
+
+    // final: dV, dK rows; each group writes half of the head dimension
+    constexpr int CD = D / 2;
+    if (ntile > 0) cta_wait(bar_done, 0, abort_flag, p.status, ERR_WAIT_TMEM_FULL);
+    tc_fence_after_sync();
+    __nv_bfloat16* dvrow = p.dv + (long long)kv * p.ld_dv + h * D + group * CD;
+    __nv_bfloat16* dkrow = p.dk + (long long)kv * p.ld_dk + h * D + group * CD;
+    if (ntile > 0) {
+      auto write = [&](uint32_t col, __nv_bfloat16* row, float mul) {
+#pragma unroll
+        for (int c = 0; c < CD; c += 32) {
+          uint32_t v[32];
+          tmem_ld_32x32b_x32(tmem_base + lane_off + col + group * CD + c, v);
+          tmem_ld_wait();
+          if (kv < p.T) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              reinterpret_cast<uint4*>(row + c)[j] =
+                  make_uint4(pack_bf16x2(__uint_as_float(v[8 * j]) * mul, __uint_as_float(v[8 * j + 1]) * mul),
+                             pack_bf16x2(__uint_as_float(v[8 * j + 2]) * mul, __uint_as_float(v[8 * j + 3]) * mul),
+                             pack_bf16x2(__uint_as_float(v[8 * j + 4]) * mul, __uint_as_float(v[8 * j + 5]) * mul),
+                             pack_bf16x2(__uint_as_float(v[8 * j + 6]) * mul, __uint_as_float(v[8 * j + 7]) * mul));
+          }
+        }
+      };
+      write(DV_COL, dvrow, 1.f);
+      write(DK_COL, dkrow, p.scale);
+    } else if (kv < p.T) {
+      // no query tile attends this key tile: its gradients are zero (the caller does not pre-zero dk / dv)
+#pragma unroll
+      for (int j = 0; j < CD / 8; ++j) {
+        reinterpret_cast<uint4*>(dvrow)[j] = make_uint4(0u, 0u, 0u, 0u);
+        reinterpret_cast<uint4*>(dkrow)[j] = make_uint4(0u, 0u, 0u, 0u);
+      }
+    }
+  }
+  __syncwarp();
+  if (tid == 0) {
+    if (*abort_flag) {
+      const uint64_t t0 = globaltimer_ns();
+      while (globaltimer_ns() - t0 < 1000000ull) __nanosleep(1000);
+    }
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  if (warp == BWD_MMA) tmem_dealloc(tmem_base, TMEM_COLS);
 }
 
 CUtensorMap qkv_map(const void* base, int T, int H, int D, long long ld, int rows) {
@@ -962,15 +1285,15 @@ void fwd_impl(const AttnArgs& a) {
 
 template <int D>
 void bwd_impl(const AttnArgs& a) {
-  constexpr int NS = D / 64;
-  const int smem = 2 * NS * 128 * 128 + 6 * NS * 64 * 128 + (D == 128 ? 1 : 2) * 128 * 128 + 64 * D * 4 + 6 * 64 * 4 + 128 + 1024;
+  const int smem = (D == 128 ? 2 * 2 * 128 * 128 + 6 * 2 * 64 * 128 + 128 * 128 : 2 * 128 * 128 + 2 * BWD64_QB * 64 * 128 + 3 * 128 * 128) +
+                   64 * D * 4 + 12 * 64 * 4 + 256 + 1024;
   CUtensorMap tq = qkv_map(a.q, a.T, a.H, D, a.ld_q, 64);
   CUtensorMap tk = qkv_map(a.k, a.T, a.H, D, a.ld_k, 128);
   CUtensorMap tv = qkv_map(a.v, a.T, a.H, D, a.ld_v, 128);
   CUtensorMap tdo = qkv_map(a.d_o, a.T, a.H, D, a.ld_do, 64);
   CUtensorMap tdq = make_tmap_3d(a.dq_acc, TmapDtype::F32, (uint64_t)D, (uint64_t)a.T, (uint64_t)a.H,
                                  (uint64_t)a.ld_dq * 4, (uint64_t)D * 4, (uint32_t)D, 64, false);
-  auto kern = attn_bwd_kernel<D>;
+  auto kern = D == 128 ? attn_bwd128_kernel : attn_bwd64_kernel;
   static PerDeviceOnce cfg;   // the shared-memory opt-in is a per-device attribute
   int dev = 0;
   if (cfg.pending(&dev)) { set_smem(kern, smem); cfg.done(dev); }

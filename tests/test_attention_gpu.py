@@ -174,6 +174,23 @@ def _blocked_oracle(q, k, v, ds, scale, window):
     return (o / l[..., None]).transpose(0, 1)
 
 
+@pytest.mark.parametrize("t", [64, 65, 128, 192, 250, 320, 384, 449, 830])
+@pytest.mark.parametrize("d", [128, 64])
+def test_attention_backward_tiles_in_turn(t, d):
+    """One to thirteen query tiles a key tile: first and last turns of the buffers (two groups of warps, three sets of scores, three or six
+    of queries), and how the report at the end finds each of them."""
+    from ml_experiments_b200.ops import attention as A
+
+    q, k, v, ds, de = _setup(t, 2, d, t, seed=t)
+    dy = torch.randn(t, 2, d, device="cuda").bfloat16()
+    grads = []
+    for fn, dt in ((lambda *x: A.flash_attention(*x, ds, de, 0.12, 0), torch.bfloat16), (lambda *x: A.attention_reference(*x, ds, 0.12), torch.float32)):
+        ins = [u.detach().to(dt).requires_grad_() for u in (q, k, v)]
+        grads.append(torch.autograd.grad(fn(*ins), ins, dy.to(dt)))
+    for got, want in zip(*grads):
+        assert ((got.float() - want).norm() / want.norm()).item() < 1.5e-2     # bf16 probabilities and results
+
+
 @pytest.mark.parametrize("t,starts,window", [(64, [0], 0), (200, [0], 0), (513, [0, 70, 190, 333], 0), (1500, [0, 900], 0),
                                              (1500, [0], 3)])
 @pytest.mark.parametrize("rising", [False, True])
