@@ -15,8 +15,7 @@ from torch import Tensor
 
 from ..ops import fused as Fz
 from ..ops import gemm as G
-from ..ops.attention import flash_attention_backward, flash_attention_forward
-from ..ops.runtime import ops
+from ..ops.runtime import add_launches, ops, status
 from ..utils.shadow import shadow_of
 
 EPS = Fz.BF16_EPS
@@ -24,6 +23,10 @@ EPS = Fz.BF16_EPS
 
 class _Saved:
     __slots__ = ("x_in", "x_mix", "xn", "qkv", "qkvp", "y", "lse", "x_a", "xn2", "h", "skip", "skip_idx")
+
+
+# Kernels of the operators that issue a block's (``runtime`` counts one a call).
+_BLOCK_FWD, _BLOCK_FWD_ATTN, _MLP_BWD, _ATTN_BWD = 4, 8, 5, 8
 
 
 def _wgrad(dy: Tensor, x: Tensor, out_shape, out: Tensor | None = None) -> Tensor:
@@ -63,6 +66,7 @@ def _forward_backward(model, input_seq: Tensor, target_seq: Tensor, swb: int, ne
             break
     saved: list[_Saved] = []
     skips: list[tuple[int, Tensor]] = []
+    st = status(dev)
     x = x0
     for i, blk in enumerate(model.blocks):
         s = _Saved()
@@ -72,22 +76,16 @@ def _forward_backward(model, input_seq: Tensor, target_seq: Tensor, swb: int, ne
         if i >= enc:
             s.skip_idx, s.skip = skips.pop()
             skip_w = model.skip_weights[i - enc:i - enc + 1]
-        s.x_mix, s.xn = Fz.mix_norm(x, x0, blk.lambdas, s.skip, skip_w, EPS)
-        if blk.attn is not None:
-            a = blk.attn
-            s.qkv = G.gemm(s.xn, w16(a.qkv_w).view(3 * HD, C))
-            s.qkvp = torch.empty_like(s.qkv)
-            ve = ves[ve_map[i]] if ve_map[i] is not None else None
-            o.qkv_post_fwd(s.qkv, ve, a.lambdas, cos, sin, s.qkvp, H, D, EPS)
-            q4 = s.qkvp.view(T, 3, H, D)
-            s.y, s.lse = flash_attention_forward(q4[:, 0], q4[:, 1], q4[:, 2], doc_start, doc_end, a.attn_scale, windows[i])
-            s.x_a = G.gemm(s.y.view(T, HD), w16(a.c_proj.weight), epilogue=G.EPI_AXPBY, aux=s.x_mix, beta=1.0)
+        mlp, a = blk.mlp, blk.attn
+        if a is not None:
+            attn = (w16(a.qkv_w).view(3 * HD, C), a.lambdas, ves[ve_map[i]] if ve_map[i] is not None else None, cos, sin, w16(a.c_proj.weight))
         else:
-            s.qkv = s.qkvp = s.y = s.lse = None
-            s.x_a = s.x_mix
-        s.xn2 = Fz.rmsnorm(s.x_a, EPS)
-        s.h = G.gemm(s.xn2, w16(blk.mlp.c_fc.weight), epilogue=G.EPI_RELU2)
-        x = G.gemm(s.h, w16(blk.mlp.c_proj.weight), epilogue=G.EPI_AXPBY, aux=s.x_a, beta=1.0)
+            attn = (None,) * 6
+        x, s.x_mix, s.xn, s.x_a, s.xn2, s.h, *rest = o.gpt_block_fwd(
+            x, x0, s.skip, skip_w, blk.lambdas, *attn, w16(mlp.c_fc.weight), w16(mlp.c_proj.weight), doc_start, doc_end, H, D,
+            a.attn_scale if a is not None else 0.0, windows[i], EPS, st)
+        s.qkv, s.qkvp, s.y, s.lse = rest or (None,) * 4
+        add_launches((_BLOCK_FWD if a is None else _BLOCK_FWD_ATTN) - 1)
         if i < enc:
             skips.append((i, x))
         saved.append(s)
@@ -109,11 +107,12 @@ def _forward_backward(model, input_seq: Tensor, target_seq: Tensor, swb: int, ne
     loss_rows = Fz.softcap_ce(logits, target_seq, gl, c.softcap, c.softcap_div, 1.0, grad_s / T)
     loss = loss_rows.mean()
     if not need_grad:
-        return loss, None
+        return loss, None, None
     del logits
 
     # ------------------------------------------------------------------ backward
     grads: dict[int, Tensor] = {}
+    owners: list[Tensor] = []          # the parameters that have one
     # Optional hand-over to a distributed optimizer: ``model._grad_out`` maps id(param) -> a preallocated gradient
     # buffer (e.g. a view of a peer-mapped bucket) that the producing kernel writes directly; ``model._grad_hooks``
     # maps id(param) -> callable(param, grad) invoked as soon as that gradient is complete (the head's is at the very
@@ -131,7 +130,11 @@ def _forward_backward(model, input_seq: Tensor, target_seq: Tensor, swb: int, ne
         return torch.zeros(p.shape, dtype=torch.float32, device=dev)
 
     def put(p, g):
-        grads[id(p)] = g if id(p) not in grads else grads[id(p)] + g
+        if id(p) in grads:
+            g = grads[id(p)] + g
+        else:
+            owners.append(p)
+        grads[id(p)] = g
         hook = grad_hooks.get(id(p))
         if hook is not None:
             hook(p, grads[id(p)])
@@ -147,41 +150,40 @@ def _forward_backward(model, input_seq: Tensor, target_seq: Tensor, swb: int, ne
     dx = Fz.norm_bwd_add(dxf, x_last, None, EPS)
 
     dx0_acc = torch.zeros(T, C, dtype=torch.float32, device=dev)
-    dskip_w = torch.zeros_like(model.skip_weights)
+    # the sums of the scalar gains: two pairs a block and one a skip, cleared together
+    nb = len(model.blocks)
+    gains = torch.zeros(4 * nb + model.skip_weights.numel(), dtype=torch.float32, device=dev)
+    dskip_w = gains[4 * nb:].view_as(model.skip_weights)
     dskips: dict[int, Tensor] = {}
     ve_grads = [None] * len(model.value_embeds.embed)
     dve_wait: dict[int, Tensor] = {}
     dq_acc = None
-    for i in reversed(range(len(model.blocks))):
+    for i in reversed(range(nb)):
         blk, s = model.blocks[i], saved[i]
         if i in dskips:
             dx = dx + dskips.pop(i)
-        mlp = blk.mlp
-        dpre = G.gemm(dx, w16(mlp.c_proj.weight), b_mn=True, epilogue=G.EPI_RELU2_BWD, aux=s.h)
-        put(mlp.c_proj.weight, _wgrad(dx, s.h, mlp.c_proj.weight.shape, out_buf(mlp.c_proj.weight)))
-        dxn2 = G.gemm(dpre, w16(mlp.c_fc.weight), b_mn=True)
-        put(mlp.c_fc.weight, _wgrad(dpre, s.xn2, mlp.c_fc.weight.shape, out_buf(mlp.c_fc.weight)))
-        del dpre
-        dx_a = Fz.norm_bwd_add(dxn2, s.x_a, dx, EPS)
+        fc, pj = blk.mlp.c_fc.weight, blk.mlp.c_proj.weight
+        dx_a, g_fc, g_pj = o.gpt_mlp_bwd(dx, s.x_a, s.xn2, s.h, w16(fc), w16(pj), out_buf(fc), out_buf(pj), G.auto_split_k(*fc.shape, T),
+                                         G.auto_split_k(*pj.shape, T), EPS, st)
+        add_launches(_MLP_BWD - 1)
+        put(pj, g_pj)
+        put(fc, g_fc)
         if blk.attn is not None:
             a = blk.attn
-            dy = G.gemm(dx_a, w16(a.c_proj.weight), b_mn=True)
-            put(a.c_proj.weight, _wgrad(dx_a, s.y.view(T, HD), a.c_proj.weight.shape, out_buf(a.c_proj.weight)))
-            q4 = s.qkvp.view(T, 3, H, D)
+            wo, wq = a.c_proj.weight, a.qkv_w
             if dq_acc is None:
-                dq_acc = torch.zeros(T, H, D, dtype=torch.float32, device=dev)
-            else:
-                dq_acc.zero_()
-            dq, dk, dv = flash_attention_backward(q4[:, 0], q4[:, 1], q4[:, 2], s.y, dy.view(T, H, D), s.lse, doc_start,
-                                                  doc_end, a.attn_scale, windows[i], dq_acc)
-            dqkv = torch.empty_like(s.qkv)
+                dq_acc = torch.empty(T, H, D, dtype=torch.float32, device=dev)
             vi = ve_map[i]
             ve = ves[vi] if vi is not None else None
-            dve = torch.empty(T, HD, dtype=torch.bfloat16, device=dev) if ve is not None else None
-            dlam = torch.zeros(2, dtype=torch.float32, device=dev)
-            o.qkv_post_bwd(dq, dk, dv, s.qkv, ve, a.lambdas, cos, sin, dqkv, dve, dlam, H, D, EPS)
+            dlam = gains[4 * i:4 * i + 2]
+            dx_mix, dve, g_wq, g_wo = o.gpt_attn_bwd(
+                dx_a, s.x_mix, s.xn, s.qkv, s.qkvp, s.y, s.lse, w16(wq).view(3 * HD, C), w16(wo), a.lambdas, ve, cos, sin, doc_start, doc_end,
+                dq_acc, dlam, out_buf(wq), out_buf(wo), G.auto_split_k(3 * HD, C, T), G.auto_split_k(C, HD, T), H, D, a.attn_scale, windows[i],
+                EPS, st)
+            add_launches(_ATTN_BWD - 1)
+            put(wo, g_wo)
             put(a.lambdas, dlam)
-            if dve is not None:
+            if ve is not None:
                 # a value embedding feeds several layers: the first gradient waits for the next one and the two are
                 # summed inside one scatter; what is still waiting at the end is flushed below
                 if vi in dve_wait:
@@ -190,25 +192,19 @@ def _forward_backward(model, input_seq: Tensor, target_seq: Tensor, swb: int, ne
                     o.embed_scatter_add(idx, dve, ve_grads[vi], dve_wait.pop(vi))
                 else:
                     dve_wait[vi] = dve
-            dxn = G.gemm(dqkv, w16(a.qkv_w).view(3 * HD, C), b_mn=True)
-            put(a.qkv_w, _wgrad(dqkv, s.xn, a.qkv_w.shape, out_buf(a.qkv_w)))
-            dx_mix = Fz.norm_bwd_add(dxn, s.x_mix, dx_a, EPS)
+            put(wq, g_wq.view(wq.shape))
         else:
             dx_mix = dx_a
-        dx_prev = torch.empty_like(dx_mix)
-        dlam_b = torch.zeros(2, dtype=torch.float32, device=dev)
+        dlam_b = gains[4 * i + 2:4 * i + 4]
         # the skip gradient waiting for the layer below is added inside this kernel, before dx_prev is rounded
         add_in = dskips.pop(i - 1, None)
-        if s.skip is not None:
-            dsk = torch.empty_like(dx_mix)
-            j = i - enc
-            o.mix_bwd(dx_mix, s.x_in, x0, s.skip, blk.lambdas, model.skip_weights[j:j + 1], dx_prev, dsk, dx0_acc, dlam_b,
-                      dskip_w[j:j + 1], add_in)
+        j = i - enc
+        has_skip = s.skip is not None
+        dx, dsk = o.gpt_mix_bwd(dx_mix, s.x_in, x0, s.skip, blk.lambdas, model.skip_weights[j:j + 1] if has_skip else None, dx0_acc, dlam_b,
+                                dskip_w[j:j + 1] if has_skip else None, add_in)
+        if has_skip:
             dskips[s.skip_idx] = dsk
-        else:
-            o.mix_bwd(dx_mix, s.x_in, x0, None, blk.lambdas, None, dx_prev, None, dx0_acc, dlam_b, None, add_in)
         put(blk.lambdas, dlam_b)
-        dx = dx_prev
         saved[i] = None
     put(model.skip_weights, dskip_w)
     # embedding: x0 = rmsnorm(embed[idx]) receives the first block's input gradient plus every lambda[1] path
@@ -225,13 +221,13 @@ def _forward_backward(model, input_seq: Tensor, target_seq: Tensor, swb: int, ne
     for vi, e in enumerate(model.value_embeds.embed):
         if ve_grads[vi] is not None:
             put(e.weight, ve_grads[vi])
-    return loss, grads
+    return loss, grads, owners
 
 
 class _FusedGPTLoss(torch.autograd.Function):
     @staticmethod
     def forward(ctx, model, input_seq, target_seq, swb, need_grad, *params):
-        loss, grads = _forward_backward(model, input_seq, target_seq, swb, need_grad)
+        loss, grads, _ = _forward_backward(model, input_seq, target_seq, swb, need_grad)
         ctx.grads = grads
         ctx.params = params
         return loss
@@ -269,15 +265,13 @@ def fused_gpt_step(model, input_seq: Tensor, target_seq: Tensor, swb: int) -> Te
     """Loss of one training step with the parameter gradients written straight into ``p.grad`` (accumulated when a
     gradient is already there): what ``fused_gpt_loss(...).backward()`` produces, without the autograd node and its
     multiply of every gradient by the incoming loss gradient (which is 1 for a plain ``backward()``)."""
-    loss, grads = _forward_backward(model, input_seq, target_seq, swb, True)
+    with torch.no_grad():
+        loss, grads, owners = _forward_backward(model, input_seq, target_seq, swb, True)
     grad_out = getattr(model, "_grad_out", None) or {}
-    for p in model.parameters():
+    for p in owners:
         if not p.requires_grad:
             continue
-        g = grads.get(id(p))
-        if g is None:
-            continue
-        g = g.view(p.shape)
+        g = grads[id(p)].view(p.shape)
         buf = grad_out.get(id(p)) if p.grad is None else None
         if buf is not None and buf.data_ptr() != g.data_ptr():
             buf.copy_(g)                      # cast (if any) and hand-over in one pass
