@@ -11,6 +11,7 @@
 //            formed transposed so that Pᵀ / dSᵀ rows are owned by one thread each and feed
 //            dV += Pᵀ·dO, dK += dSᵀ·Q (TMEM-resident accumulators) and dQᵀ = Kᵀ·dSᵀ, which is
 //            added into an fp32 dQ buffer by TMA reduce-add.
+#include "../common/launch.h"
 #include "../common/per_device.h"
 #include "attn.h"
 
@@ -177,6 +178,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const bool leave = __syncthreads_or(poisoned);     // all warps or none
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  let_next_start();
+  after_previous();                                  // the set-up has run under the end of the kernel before
   if (leave) {
     if (warp == 8) tmem_dealloc(tmem_base, TMEM_COLS);
     return;
@@ -480,6 +483,9 @@ template <int D>
 __global__ void attn_delta_vec_kernel(const __nv_bfloat16* __restrict__ o, long long ld_o,
                                       const __nv_bfloat16* __restrict__ d_o, long long ld_do,
                                       float* __restrict__ delta, int T, int H) {
+  let_next_start();
+  after_previous();
+  o = fresh(o), d_o = fresh(d_o);
   constexpr int LPR = D / 8;
   const long long row = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / LPR;
   const int sub = threadIdx.x % LPR;
@@ -559,6 +565,7 @@ attn_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
+  after_previous();
   const bool poisoned = status_poisoned(p.status);
   const int tid = threadIdx.x;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
@@ -612,6 +619,7 @@ attn_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   const bool leave = __syncthreads_or(poisoned);     // all warps or none
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  let_next_start();
   if (leave) {
     if (warp == BWD_MMA) tmem_dealloc(tmem_base, TMEM_COLS);
     return;
@@ -908,6 +916,7 @@ attn_bwd64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_done + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
+  after_previous();
   const bool poisoned = status_poisoned(p.status);
   const int tid = threadIdx.x;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
@@ -960,6 +969,7 @@ attn_bwd64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   const bool leave = __syncthreads_or(poisoned);     // all warps or none
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  let_next_start();
   if (leave) {
     if (warp == BWD_MMA) tmem_dealloc(tmem_base, TMEM_COLS);
     return;
@@ -1256,7 +1266,7 @@ void fwd_launch(const AttnArgs& a, const KP& p, int items) {
   CUtensorMap tv = qkv_map(a.v, a.T, a.H, D, a.ld_v, FKV);
   auto kern = attn_fwd_kernel<D, MIXED>;
   const int grid = std::min(p.pairs + 2 * (items - p.pairs), sm_count());
-  kern<<<grid, FWD_THREADS, F::SMEM, a.stream>>>(tq, tk, tv, p);
+  launch_early(kern, grid, FWD_THREADS, F::SMEM, a.stream, tq, tk, tv, p);
   check_launch("attn_fwd launch");
 }
 
@@ -1298,7 +1308,7 @@ void bwd_impl(const AttnArgs& a) {
   int dev = 0;
   if (cfg.pending(&dev)) { set_smem(kern, smem); cfg.done(dev); }
   dim3 grid((a.T + 127) / 128, a.H);
-  kern<<<grid, BWD_THREADS, smem, a.stream>>>(tq, tk, tv, tdo, tdq, make_kp(a));
+  launch_early(kern, grid, BWD_THREADS, smem, a.stream, tq, tk, tv, tdo, tdq, make_kp(a));
   check_launch("attn_bwd launch");
 }
 
@@ -1320,8 +1330,8 @@ void attn_delta_sm100(const AttnArgs& a) {
   if (aligned) {
     const long long lanes = warps * (a.D / 8);
     const int vblocks = (int)((lanes + threads - 1) / threads);
-    if (a.D == 128) attn_delta_vec_kernel<128><<<vblocks, threads, 0, a.stream>>>(o, a.ld_o, d_o, a.ld_do, a.delta, a.T, a.H);
-    else            attn_delta_vec_kernel<64><<<vblocks, threads, 0, a.stream>>>(o, a.ld_o, d_o, a.ld_do, a.delta, a.T, a.H);
+    if (a.D == 128) launch_early(attn_delta_vec_kernel<128>, vblocks, threads, 0, a.stream, o, a.ld_o, d_o, a.ld_do, a.delta, a.T, a.H);
+    else            launch_early(attn_delta_vec_kernel<64>, vblocks, threads, 0, a.stream, o, a.ld_o, d_o, a.ld_do, a.delta, a.T, a.H);
   } else if (a.D == 128) {
     attn_delta_kernel<128><<<blocks, threads, 0, a.stream>>>(o, a.ld_o, d_o, a.ld_do, a.delta, a.T, a.H);
   } else {

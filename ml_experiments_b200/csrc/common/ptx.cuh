@@ -50,6 +50,21 @@ __device__ __forceinline__ uint32_t elect_one_sync() {
   return pred;
 }
 
+// Programmatic dependent launch: a kernel launched with that attribute may start while the one before it in the stream still runs.
+// `after_previous` waits until that one (and, as it waited itself, all before it) has ended and its writes are visible. Every block calls
+// it, before its first access to memory that another kernel writes or reads and before it ends; only a status word may be read earlier
+// (one that is set meanwhile is missed: this kernel's waits are bounded as well). `let_next_start`: once all blocks of a grid have called
+// it, blocks of the next kernel take the room that is left. A block that allocates tensor memory calls it after that: the next kernel's
+// block would hold what this one waits for, and wait for this one.
+__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// A kernel's pointer parameter, for use after `after_previous`: loads through a const restrict parameter may be moved to in front of it.
+template <typename T>
+__device__ __forceinline__ T* fresh(T* p) {
+  asm volatile("" : "+l"(p)::"memory");
+  return p;
+}
+
 // Registers per thread of a warpgroup (all four warps execute it). The shares must add up to no more than the block was
 // launched with: an allocation beyond that would wait for ever.
 template <int N>

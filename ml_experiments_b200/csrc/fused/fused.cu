@@ -3,7 +3,9 @@
 // One warp owns one row wherever a row reduction is needed; all global accesses are 16-byte vectors.
 #include "fused.h"
 
+#include "common/launch.h"
 #include "common/per_device.h"
+#include "common/ptx.cuh"
 
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
@@ -78,6 +80,9 @@ __global__ void __launch_bounds__(kRowThreads)
 mix_norm_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ x0, const bf16* __restrict__ skip,
                     const float* __restrict__ lam, const float* __restrict__ skip_w, bf16* __restrict__ x_mix,
                     bf16* __restrict__ xn, int R, int C, float eps) {
+  let_next_start();
+  after_previous();
+  x = fresh(x), x0 = fresh(x0), skip = fresh(skip), lam = fresh(lam), skip_w = fresh(skip_w);
   const int row = (blockIdx.x * kRowThreads + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (row >= R) return;
@@ -130,6 +135,9 @@ template <int NCH>
 __global__ void __launch_bounds__(kRowThreads)
 norm_bwd_add_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, const bf16* __restrict__ dres,
                     bf16* __restrict__ out, int R, int C, float eps) {
+  let_next_start();
+  after_previous();
+  dy = fresh(dy), x = fresh(x), dres = fresh(dres);
   const int row = (blockIdx.x * kRowThreads + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (row >= R) return;
@@ -176,6 +184,9 @@ mix_bwd_kernel(const bf16* __restrict__ dmix, const bf16* __restrict__ x, const 
                const bf16* __restrict__ skip, const float* __restrict__ lam, const float* __restrict__ skip_w,
                bf16* __restrict__ dx, bf16* __restrict__ dskip, float* __restrict__ dx0_acc, float* __restrict__ dlam,
                float* __restrict__ dskip_w, const bf16* __restrict__ dx_add, int R, int C) {
+  let_next_start();
+  after_previous();
+  dmix = fresh(dmix), x = fresh(x), x0 = fresh(x0), skip = fresh(skip), lam = fresh(lam), skip_w = fresh(skip_w), dx_add = fresh(dx_add);
   __shared__ float red[3][kRowThreads / 32];
   const int warp_in_block = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -259,6 +270,9 @@ __global__ void __launch_bounds__(256)
 qkv_post_fwd_kernel(const bf16* __restrict__ qkv, const bf16* __restrict__ ve, const float* __restrict__ lam,
                     const float* __restrict__ cs, const float* __restrict__ sn, bf16* __restrict__ out, int T, int H,
                     float eps) {
+  let_next_start();
+  after_previous();
+  qkv = fresh(qkv), ve = fresh(ve), lam = fresh(lam), cs = fresh(cs), sn = fresh(sn);
   constexpr int LPR = D / 16;
   const long long row = ((long long)blockIdx.x * 256 + threadIdx.x) / LPR;
   const int sub = threadIdx.x % LPR;
@@ -313,6 +327,9 @@ qkv_post_bwd_kernel(const float* __restrict__ dq, const bf16* __restrict__ dk, c
                     const bf16* __restrict__ qkv, const bf16* __restrict__ ve, const float* __restrict__ lam,
                     const float* __restrict__ cs, const float* __restrict__ sn, bf16* __restrict__ dqkv,
                     bf16* __restrict__ dve, float* __restrict__ dlam, int T, int H, float eps) {
+  let_next_start();
+  after_previous();
+  dq = fresh(dq), dk = fresh(dk), dv = fresh(dv), qkv = fresh(qkv), ve = fresh(ve), lam = fresh(lam), cs = fresh(cs), sn = fresh(sn);
   constexpr int LPR = D / 16;
   __shared__ float red[2][8];
   const int sub = threadIdx.x % LPR;
@@ -810,14 +827,14 @@ void rmsnorm_fwd(const void* x, void* y, int R, int C, float eps, cudaStream_t s
 
 void mix_norm_fwd(const void* x, const void* x0, const void* skip, const float* lam, const float* skip_w,
                   void* x_mix, void* xn, int R, int C, float eps, cudaStream_t s) {
-  DISPATCH_NCH(C, (mix_norm_fwd_kernel<N_><<<row_blocks(R), kRowThreads, 0, s>>>(
+  DISPATCH_NCH(C, (launch_early(mix_norm_fwd_kernel<N_>, row_blocks(R), kRowThreads, 0, s,
                       (const bf16*)x, (const bf16*)x0, (const bf16*)skip, lam, skip_w, (bf16*)x_mix, (bf16*)xn, R, C, eps)));
   check("mix_norm_fwd");
 }
 
 void norm_bwd_add(const void* dy, const void* x, const void* dres, void* out, int R, int C, float eps,
                   cudaStream_t s) {
-  DISPATCH_NCH(C, (norm_bwd_add_kernel<N_><<<row_blocks(R), kRowThreads, 0, s>>>((const bf16*)dy, (const bf16*)x,
+  DISPATCH_NCH(C, (launch_early(norm_bwd_add_kernel<N_>, row_blocks(R), kRowThreads, 0, s, (const bf16*)dy, (const bf16*)x,
                                                                                  (const bf16*)dres, (bf16*)out, R, C, eps)));
   check("norm_bwd_add");
 }
@@ -826,7 +843,7 @@ void mix_bwd(const void* dmix, const void* x, const void* x0, const void* skip, 
              const float* skip_w, void* dx, void* dskip, float* dx0_acc, float* dlam, float* dskip_w, const void* dx_add,
              int R, int C, cudaStream_t s) {
   const int blocks = 148 * 4;
-  DISPATCH_NCH(C, (mix_bwd_kernel<N_><<<blocks, kRowThreads, 0, s>>>((const bf16*)dmix, (const bf16*)x, (const bf16*)x0,
+  DISPATCH_NCH(C, (launch_early(mix_bwd_kernel<N_>, blocks, kRowThreads, 0, s, (const bf16*)dmix, (const bf16*)x, (const bf16*)x0,
                                                                     (const bf16*)skip, lam, skip_w, (bf16*)dx,
                                                                     (bf16*)dskip, dx0_acc, dlam, dskip_w, (const bf16*)dx_add, R, C)));
   check("mix_bwd");
@@ -837,8 +854,8 @@ void qkv_post_fwd(const void* qkv, const void* ve, const float* lam, const float
   const long long rows = (long long)T * 3 * H;
   const int rpb = 256 / (D / 16);
   const int blocks = (int)((rows + rpb - 1) / rpb);
-  if (D == 128) qkv_post_fwd_kernel<128><<<blocks, 256, 0, s>>>((const bf16*)qkv, (const bf16*)ve, lam, cos, sin, (bf16*)out, T, H, eps);
-  else if (D == 64) qkv_post_fwd_kernel<64><<<blocks, 256, 0, s>>>((const bf16*)qkv, (const bf16*)ve, lam, cos, sin, (bf16*)out, T, H, eps);
+  if (D == 128) launch_early(qkv_post_fwd_kernel<128>, blocks, 256, 0, s, (const bf16*)qkv, (const bf16*)ve, lam, cos, sin, (bf16*)out, T, H, eps);
+  else if (D == 64) launch_early(qkv_post_fwd_kernel<64>, blocks, 256, 0, s, (const bf16*)qkv, (const bf16*)ve, lam, cos, sin, (bf16*)out, T, H, eps);
   else throw std::runtime_error("qkv_post: head_dim must be 64 or 128");
   check("qkv_post_fwd");
 }
@@ -850,8 +867,8 @@ void qkv_post_bwd(const float* dq, const void* dk, const void* dv, const void* q
   const int rpb = 256 / (D / 16);
   int blocks = (int)((rows + rpb - 1) / rpb);
   if (blocks > 148 * 4) blocks = 148 * 4;     // 64 registers: four resident blocks of 256 threads per SM
-  if (D == 128) qkv_post_bwd_kernel<128><<<blocks, 256, 0, s>>>(dq, (const bf16*)dk, (const bf16*)dv, (const bf16*)qkv, (const bf16*)ve, lam, cos, sin, (bf16*)dqkv, (bf16*)dve, dlam, T, H, eps);
-  else if (D == 64) qkv_post_bwd_kernel<64><<<blocks, 256, 0, s>>>(dq, (const bf16*)dk, (const bf16*)dv, (const bf16*)qkv, (const bf16*)ve, lam, cos, sin, (bf16*)dqkv, (bf16*)dve, dlam, T, H, eps);
+  if (D == 128) launch_early(qkv_post_bwd_kernel<128>, blocks, 256, 0, s, dq, (const bf16*)dk, (const bf16*)dv, (const bf16*)qkv, (const bf16*)ve, lam, cos, sin, (bf16*)dqkv, (bf16*)dve, dlam, T, H, eps);
+  else if (D == 64) launch_early(qkv_post_bwd_kernel<64>, blocks, 256, 0, s, dq, (const bf16*)dk, (const bf16*)dv, (const bf16*)qkv, (const bf16*)ve, lam, cos, sin, (bf16*)dqkv, (bf16*)dve, dlam, T, H, eps);
   else throw std::runtime_error("qkv_post: head_dim must be 64 or 128");
   check("qkv_post_bwd");
 }

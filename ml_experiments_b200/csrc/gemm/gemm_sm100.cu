@@ -118,6 +118,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   }
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  let_next_start();
+  after_previous();                                  // the set-up above has run under the end of the kernel before
   if (leave) {
     if (PAIR) cluster_sync();                        // the word has been read
     if (warp == 1) {
@@ -450,12 +452,14 @@ void launch(const GemmArgs& a, const KParams& kp, const CUtensorMap& tA, const C
   cfg.blockDim = dim3(threads(PAIR));
   cfg.dynamicSmemBytes = L::kTotal;
   cfg.stream = a.stream;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = PAIR + 1;
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = PAIR ? 1 : 0;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = PAIR + 1;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = PAIR ? 2 : 1;
   cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tA, tB, tC, tX, kp);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) throw std::runtime_error(std::string("gemm launch: ") + cudaGetErrorString(e));
