@@ -84,8 +84,40 @@ __device__ __forceinline__ float ld(const float* p, long long i) { return p[i]; 
 __device__ __forceinline__ float ld(const bf16* p, long long i) { return __bfloat162float(p[i]); }
 __device__ __forceinline__ void st(float* p, long long i, float v) { p[i] = v; }
 __device__ __forceinline__ void st(bf16* p, long long i, float v) { p[i] = __float2bfloat16_rn(v); }
-__device__ __forceinline__ float sigmoidf(float x) { return 1.f / (1.f + __expf(-x)); }
-__device__ __forceinline__ float softplusf(float x) { return x > 20.f ? x : log1pf(__expf(x)); }
+
+// Softplus and sigmoid without a branch, so that those of several steps and channels are under way at once (a division and log1pf
+// have branches). Both from t = exp(-|x|); quotients are the hardware's approximate reciprocal and one Newton step on the exact
+// remainder, which also takes in the rounding of the denominator.
+__device__ __forceinline__ float rcp_approx(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float sigmoid_of(float x, float t) {
+  const float r = rcp_approx(1.f + t), n = x < 0.f ? t : 1.f, y = n * r;          // n / (1 + t)
+  return fmaf(fmaf(-y, t, n - y), r, y);
+}
+// softplus(x) = max(x, 0) + log(1 + t), and log(1 + t) = 2 atanh(s) = 2 (s + s^3 / 3 + s^5 / 5 + ...) with s = t / (2 + t) <= 1/3: what
+// is left out of the series is 1.4e-9 of it. Root mean square error against 64 bits, |x| <= 5: 6.0e-8, of the sigmoid 5.7e-8 (log1pf of
+// __expf and the division: 6.2e-8 both). Results below 2^-126 are 0. Backward, 8 x 4096 x 2048: 1.82 -> 1.76 ms.
+__device__ __forceinline__ float softplus_of(float x, float t) {
+  const float r = rcp_approx(2.f + t), s0 = t * r, s = fmaf(fmaf(-s0, t, fmaf(-2.f, s0, t)), r, s0), q = s * s;
+  float p = fmaf(q, 1.f / 15, 1.f / 13);
+  p = fmaf(q, p, 1.f / 11);
+  p = fmaf(q, p, 1.f / 9);
+  p = fmaf(q, p, 1.f / 7);
+  p = fmaf(q, p, 1.f / 5);
+  p = fmaf(q, p, 1.f / 3);
+  return fmaxf(x, 0.f) + fmaf(-s, fmaf(-2.f * q, p, t), t);          // 2 s = t - s t
+}
+__device__ __forceinline__ float exp_minus_abs(float x) { return ex2(-LOG2E * fabsf(x)); }
+__device__ __forceinline__ float sigmoidf(float x) { return sigmoid_of(x, exp_minus_abs(x)); }
+__device__ __forceinline__ float softplusf(float x) { return softplus_of(x, exp_minus_abs(x)); }
+__device__ __forceinline__ float softplusf(float x, float& derivative) {
+  const float t = exp_minus_abs(x);
+  derivative = sigmoid_of(x, t);
+  return softplus_of(x, t);
+}
 
 template <int QS>
 struct FwdSmem {
@@ -205,8 +237,9 @@ s6_fwd_kernel(const bf16* __restrict__ u, const DT* __restrict__ delta, const fl
 //
 // Bound: one exponential per state and step (SFU: 8 cycles per warp instruction), 0.24 ms of 8 x 4096 x 2048 x 16; the
 // softplus and the gate add a quarter to it. Shared memory takes 3 vector loads and 3/4 of a shuffle per warp step.
-// Measured: 0.547 ms there (0.721 ms in the general kernel: a warp per two states of 32 channels, partial sums in shared memory),
-// 3 x 1531 x 1024: 0.110 ms (0.170 ms).
+// Measured, with the states stored: 0.611 ms there (0.661 ms with log1pf, divisions and a loop over the pieces to copy), 1 x 4096 x
+// 2048: 0.223 ms (0.252 ms). The general kernel (a warp per two states of 32 channels, partial sums in shared memory) takes 0.17 ms
+// for 3 x 1531 x 1024, this one 0.112.
 constexpr int PC = 16;   // channels per block of the forward
 
 template <typename DT>
@@ -283,32 +316,24 @@ s6_fwd_pipe_kernel(const bf16* __restrict__ u, const DT* __restrict__ delta, con
   const float bias = (dok && delta_bias) ? delta_bias[d] : 0.f;
   const float dsk = (dok && Dv) ? Dv[d] : 0.f;
 
+  // a thread copies one 16-byte piece of each pair of 32-byte rows and of B and C; where there are 128, half of that
+  const int row = (tid & 63) >> 2, piece = tid & 3, ch = (piece & 1) * 8;
+  const bool first = NT == 64 || tid < 64, second = NT == 64 || tid >= 64;
   auto issue = [&](int tile) {
     if (tile < nsub) {
       FwdRaw<DT>& r = raw[tile % STAGES];
-      const int t0 = tile * SUB;
-      constexpr int DPR = PC * (int)sizeof(DT) / 16, ND = SUB * DPR, N16 = SUB * 2, NBC = SUB * NS / 4;
-      const int total = ND + N16 + 2 * NBC + (z ? N16 : 0);
-      for (int i = tid; i < total; i += NT) {
-        int j = i;
-        if (j < ND) {
-          const int row = j / DPR, part = j % DPR, per = 16 / (int)sizeof(DT), ch = d0 + part * per;
-          const int ok = (t0 + row < L && ch < Din) ? 16 : 0;
-          cp_async16(&r.delta[row][part * per], delta + ((long long)b * L + min(t0 + row, L - 1)) * Din + min(ch, Din - per), ok);
-          continue;
-        }
-        j -= ND;
-        if (j < 2 * NBC) {
-          const int row = (j % NBC) / 4, part = j % 4;
-          const float* src = (j < NBC ? Bm : Cm) + ((long long)b * L + min(t0 + row, L - 1)) * NS + part * 4;
-          cp_async16(j < NBC ? &r.B[row][part * 4] : &r.C[row][part * 4], src, t0 + row < L ? 16 : 0);
-          continue;
-        }
-        j -= 2 * NBC;
-        const int row = (j % N16) / 2, ch = d0 + (j % 2) * 8;
-        const int ok = (t0 + row < L && ch < Din) ? 16 : 0;
-        cp_async16(j < N16 ? &r.u[row][(j % 2) * 8] : &r.z[row][(j % 2) * 8],
-                   (j < N16 ? u : z) + ((long long)b * L + min(t0 + row, L - 1)) * Din + min(ch, Din - 8), ok);
+      const bool rok = tile * SUB + row < L;
+      const long long bt = (long long)b * L + min(tile * SUB + row, L - 1), off = bt * Din + min(d0 + ch, Din - 8);
+      const int n16 = (rok && d0 + ch < Din) ? 16 : 0;
+      if (first) {
+        if (sizeof(DT) == 4) cp_async16(&r.delta[row][piece * 4], delta + bt * Din + min(d0 + piece * 4, Din - 4), (rok && d0 + piece * 4 < Din) ? 16 : 0);
+        else if (piece < 2) cp_async16(&r.delta[row][ch], delta + off, n16);
+        cp_async16(&r.B[row][piece * 4], Bm + bt * NS + piece * 4, rok ? 16 : 0);
+      }
+      if (second) {
+        if (piece < 2) cp_async16(&r.u[row][ch], u + off, n16);
+        else if (z) cp_async16(&r.z[row][ch], z + off, n16);
+        cp_async16(&r.C[row][piece * 4], Cm + bt * NS + piece * 4, rok ? 16 : 0);
       }
     }
     cp_async_commit();       // also when empty: the groups are counted
@@ -321,17 +346,18 @@ s6_fwd_pipe_kernel(const bf16* __restrict__ u, const DT* __restrict__ delta, con
     __syncthreads();         // the tile is visible to all, and nobody works on the one before it any more
     issue(tile + STAGES - 1);
     const FwdRaw<DT>& r = raw[tile % STAGES];
-    float uu[KS], zz[KS];
+    float uu[KS], zz[KS], dt[KS];
 #pragma unroll
     for (int k = 0; k < KS; ++k) {
       const int t = k * G + g;
-      float dt = (float)r.delta[t][c];
-      if (softplus) dt = softplusf(dt + bias);
-      if (t0 + t >= L) dt = 0.f;
+      dt[k] = (float)r.delta[t][c];
       uu[k] = __bfloat162float(r.u[t][c]);
       zz[k] = z ? __bfloat162float(r.z[t][c]) : 0.f;
-      step[t][c] = make_float2(dt, dt * uu[k]);
+      if (softplus) dt[k] = softplusf(dt[k] + bias);
+      if (t0 + t >= L) dt[k] = 0.f;
     }
+#pragma unroll
+    for (int k = 0; k < KS; ++k) step[k * G + g][c] = make_float2(dt[k], dt[k] * uu[k]);
     __syncwarp();
     if (state && dok) {
       float o[QS];
@@ -461,8 +487,8 @@ s6_bwd_kernel(const bf16* __restrict__ u, const DT* __restrict__ delta, const fl
       sp[j] = 1.f;
       if (softplus) {
         const float raw = dtv + bias;
-        sp[j] = raw > 20.f ? 1.f : sigmoidf(raw);
-        dtv = ok ? softplusf(raw) : 0.f;
+        dtv = softplusf(raw, sp[j]);
+        if (!ok) dtv = 0.f;
       }
       float g = ok ? __bfloat162float(dout[off]) : 0.f;
       if (z && ok) {
@@ -612,26 +638,50 @@ struct RawTile {
   float st[4][PC][4];   // the state checkpoint of the tile: [group of four states][channel][state in group]
 };
 
-// Backward of the pipelined form. Block = 16 channels, two warps of 8 channels x 4 groups of 4 states, one tile of 16
-// steps at a time from the last to the first, the next tile copied by cp.async meanwhile. A tile is walked forwards once
+// Two channels' values as a packed pair, and back to memory
+__device__ __forceinline__ uint64_t ld_pair(const float* p) { return *reinterpret_cast<const uint64_t*>(p); }
+__device__ __forceinline__ uint64_t ld_pair(const bf16* p) {
+  const float2 v = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p));
+  return f2_pack(v.x, v.y);
+}
+__device__ __forceinline__ void st_pair(float* p, uint64_t v) { *reinterpret_cast<uint64_t*>(p) = v; }
+__device__ __forceinline__ void st_pair(bf16* p, uint64_t v) {
+  float x, y;
+  f2_unpack(v, x, y);
+  *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(x, y);
+}
+// What the lane `m` away sends of its (a, b), added to this lane's: b of both where `up`, else a.
+__device__ __forceinline__ uint64_t pair_exchange(uint64_t a, uint64_t b, bool up, int m) {
+  return f2_add(up ? b : a, __shfl_xor_sync(0xffffffffu, up ? a : b, m));
+}
+
+// Backward of the pipelined form. Block = 16 channels, two warps of 4 pairs of channels x 8 groups of 2 states, one tile of 16
+// steps at a time from the last to the first, the next tile copied by cp.async meanwhile. All arithmetic is on packed pairs of
+// neighbouring channels, so what depends on the channel and step alone (dt, dt u, dL/dy) is a pair as it lies in shared memory;
+// B and C, the same for all channels, are laid out there twice. A tile is walked forwards once
 // to get the states at its steps 4, 8 and 12, then four steps at a time: their decays and states are formed and kept in
 // registers (28 exponentials per 16 steps instead of 32 or a register per step), then the adjoint runs back over them.
-// Sums over channels (dB, dC: 8 values a step) and over states (d dt, d u: of four steps together) are halving
-// exchanges, 7 + 1.5 shuffles per warp step; dB / dC of the two warps meet in shared memory at the end of the tile and
+// Sums over channels (dB, dC: 4 values a step) are halving exchanges of 3 shuffles a step; sums over states (d dt, d u of four
+// steps: 8 pairs, one for each group) 3.5. dB / dC of the two warps meet in shared memory at the end of the tile and
 // those of the two blocks of a 32-channel partial sum in memory: two atomic additions to a cleared value, the same in either
 // order. At 8 x 4096 x 2048 that clears 268 MB and adds to it twice where blocks of 32 channels stored it once.
-// Blocks of two warps spread evenly (8 x 2048 channels: 6.9 of 7 on every SM) at 128 registers a thread (with fp32 delta 12
-// bytes are spilled).
-// Bound: issue slots (134 warp instructions per 128 state steps) and shared memory (31 wavefronts). Measured, 8 x 4096 x 2048:
-// 1.93 ms (1.97 ms with blocks of 32 channels; 4 states of 2 channels a thread: 1.82 ms there, but 0.56 instead of 0.43 ms at
-// 3 x 1531 x 1024, where seven warps a multiprocessor do not cover the latencies; 2.37 ms in the
-// general kernel with its inputs copied one tile ahead), 1 x 4096 x 2048: 1.03 ms (1.62 ms).
+// Blocks of two warps spread evenly (8 x 2048 channels: 6.9 of 7 on every SM) at 128 registers a thread; the states in front of steps
+// 0, 4 and 8 wait in shared memory, where they would be spilled. Loads of shared memory stand in front of the stores of their
+// section: nothing can move them there.
+// Bound: issue slots (0.6 of them used on average, four warps on two of an SM's schedulers and three on the others; 117 warp
+// instructions per 128 state steps) and, with fewer warps, the chain of one (334 cycles a step). Measured, 8 x 4096 x 2048:
+// 1.68 ms (1.86 ms with states in pairs: a channel and four states a thread, 141 instructions; 1.89 ms with the loads between the
+// stores and lanes in the plain order), 1 x 4096 x 2048: 0.72 ms (1.02 ms), 3 x 1531 x 1024: 0.288 ms (0.397 ms).
 constexpr int BWD_NT = 64;
 
 template <typename DT>
 struct BwdPipe {
   RawTile<DT> raw[2];
-  float4 step[SUB][PC];         // {dt, u, dy, d softplus}
+  ulonglong2 dt[SUB][PC / 2];   // {dt, dt u} of a pair of channels
+  ulonglong2 gy[SUB][PC / 2];   // {dL/dy, u}
+  uint64_t sp[SUB][PC / 2];     // d softplus
+  uint64_t B[SUB][NS], C[SUB][NS];   // each value twice
+  ulonglong2 h[3][BWD_NT];      // a thread's states in front of steps 0, 4 and 8
   float part[2][SUB][32];       // [warp][step][dB of 16 states, dC of 16 states]
 };
 
@@ -644,24 +694,26 @@ s6_bwd_pipe_kernel(const bf16* __restrict__ u, const DT* __restrict__ delta, con
                    DT* __restrict__ ddelta, float* __restrict__ dA, float* __restrict__ dB_part,
                    float* __restrict__ dC_part, float* __restrict__ dD, bf16* __restrict__ dz,
                    float* __restrict__ ddelta_bias, int L, int Din) {
-  constexpr int NT = BWD_NT, G = 4, CW = 8;
+  constexpr int NT = BWD_NT;
   extern __shared__ __align__(16) unsigned char s6_dyn_smem[];
   BwdPipe<DT>& s = *reinterpret_cast<BwdPipe<DT>*>(s6_dyn_smem);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int g = lane >> 3, c = warp * CW + (lane & 7);
+  // group of two states, pair of channels. A 16-byte load of shared memory takes two cycles instead of four where lanes whose number
+  // differs in bit 0, or in bit 1, read the same: bit 0 is of the pair (B, C) and bit 1 of the group (what depends on the channel).
+  const int g = (lane >> 1 & 1) | (lane >> 2 & 6), cp = warp * 4 + ((lane & 1) | (lane >> 1 & 2)), c = 2 * cp;
   const int b = blockIdx.y, d0 = blockIdx.x * PC, d = d0 + c, nblk = (Din + CB - 1) / CB;
-  const bool dok = d < Din;
+  const bool dok = d < Din;                                             // (Din is even)
   const int nsub = (L + SUB - 1) / SUB;
   uint64_t ar[2], a2[2], cr[2] = {0, 0}, dAa[2] = {0, 0};
 #pragma unroll
-  for (int p = 0; p < 2; ++p) {
-    const long long o = (long long)d * NS + g * 4 + 2 * p;
-    ar[p] = dok ? f2_pack(A[o], A[o + 1]) : 0;
-    a2[p] = f2_mul(ar[p], f2_pack(LOG2E, LOG2E));
+  for (int n = 0; n < 2; ++n) {
+    const long long o = (long long)d * NS + 2 * g + n;
+    ar[n] = dok ? f2_pack(A[o], A[o + NS]) : 0;
+    a2[n] = f2_mul(ar[n], f2_pack(LOG2E, LOG2E));
   }
-  const float bias = (dok && delta_bias) ? delta_bias[d] : 0.f;
-  const float dsk = (dok && Dv) ? Dv[d] : 0.f;
-  float dDa = 0.f, dbias = 0.f;
+  const float2 bias = (dok && delta_bias) ? make_float2(delta_bias[d], delta_bias[d + 1]) : make_float2(0.f, 0.f);
+  const uint64_t dsk = (dok && Dv) ? f2_pack(Dv[d], Dv[d + 1]) : 0;
+  uint64_t acc = 0;                                                     // groups 0-3: d delta_bias, 4-7: dD
 
   // a thread copies one 16-byte piece of each pair of 32-byte rows and of B, C and the state checkpoint
   const int row = tid >> 2, piece = tid & 3;
@@ -689,138 +741,168 @@ s6_bwd_pipe_kernel(const bf16* __restrict__ u, const DT* __restrict__ delta, con
     __syncthreads();           // the tile is visible, and the other buffer and `part` are free
     if (tile > 0) issue(tile - 1, buf ^ 1);
     const RawTile<DT>& r = s.raw[buf];
+    // (all loads in front of the first store: neither compiler nor hardware can know that they do not meet)
+    uint64_t in[2][5];
 #pragma unroll
-    for (int k = 0; k < SUB / G; ++k) {
-      const int t = k * G + g;
-      const bool ok = dok && t0 + t < L;
-      float dt = (float)r.delta[t][c], sp = 1.f;
-      if (softplus) {
-        const float x = dt + bias;
-        sp = x > 20.f ? 1.f : sigmoidf(x);
-        dt = softplusf(x);
-      }
-      float gy = __bfloat162float(r.dout[t][c]);
-      if (z) {
-        const float zv = __bfloat162float(r.z[t][c]), sg = sigmoidf(zv);
-        if (dz && ok) dz[((long long)b * L + t0 + t) * Din + d] = __float2bfloat16_rn(gy * __bfloat162float(r.yp[t][c]) * sg * (1.f + zv * (1.f - sg)));
-        gy *= zv * sg;
-      }
-      s.step[t][c] = ok ? make_float4(dt, __bfloat162float(r.u[t][c]), gy, sp) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int k = 0; k < 2; ++k) {
+      const int t = k * 8 + g;
+      in[k][0] = ld_pair(&r.delta[t][c]), in[k][1] = ld_pair(&r.u[t][c]), in[k][2] = ld_pair(&r.dout[t][c]);
+      if (z) in[k][3] = ld_pair(&r.z[t][c]), in[k][4] = ld_pair(&r.yp[t][c]);
     }
-    __syncwarp();
-    uint64_t hc[4][2];         // states in front of steps 0, 4, 8, 12
+    const float4 vb = *reinterpret_cast<const float4*>(&r.B[row][piece * 4]), vc = *reinterpret_cast<const float4*>(&r.C[row][piece * 4]);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int t = k * 8 + g;
+      const bool ok = dok && t0 + t < L;
+      float dt[2], sp[2] = {1.f, 1.f}, uu[2], gy[2];
+      f2_unpack(in[k][0], dt[0], dt[1]);
+      f2_unpack(in[k][1], uu[0], uu[1]);
+      f2_unpack(in[k][2], gy[0], gy[1]);
+      if (softplus) {
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          dt[q] = softplusf(dt[q] + (q ? bias.y : bias.x), sp[q]);
+        }
+      }
+      if (z) {
+        float zv[2], yp[2], o[2];
+        f2_unpack(in[k][3], zv[0], zv[1]);
+        f2_unpack(in[k][4], yp[0], yp[1]);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const float sg = sigmoidf(zv[q]);
+          o[q] = gy[q] * yp[q] * sg * (1.f + zv[q] * (1.f - sg));
+          gy[q] *= zv[q] * sg;
+        }
+        if (dz && ok) st_pair(&dz[((long long)b * L + t0 + t) * Din + d], f2_pack(o[0], o[1]));
+      }
+      const ulonglong2 e1 = make_ulonglong2(f2_pack(dt[0], dt[1]), f2_pack(dt[0] * uu[0], dt[1] * uu[1]));
+      const ulonglong2 e2 = make_ulonglong2(f2_pack(gy[0], gy[1]), f2_pack(uu[0], uu[1]));
+      s.dt[t][cp] = ok ? e1 : make_ulonglong2(0, 0);
+      s.gy[t][cp] = ok ? e2 : make_ulonglong2(0, 0);
+      s.sp[t][cp] = f2_pack(sp[0], sp[1]);
+    }
     {
-      const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(&r.st[g][c][0]);
-      hc[0][0] = v.x, hc[0][1] = v.y;
+      float4* ob = reinterpret_cast<float4*>(&s.B[row][piece * 4]);
+      float4* oc = reinterpret_cast<float4*>(&s.C[row][piece * 4]);
+      ob[0] = make_float4(vb.x, vb.x, vb.y, vb.y), ob[1] = make_float4(vb.z, vb.z, vb.w, vb.w);
+      oc[0] = make_float4(vc.x, vc.x, vc.y, vc.y), oc[1] = make_float4(vc.z, vc.z, vc.w, vc.w);
+    }
+    __syncthreads();
+    uint64_t h[2];
+    {
+      const float2 v0 = *reinterpret_cast<const float2*>(&r.st[g >> 1][c][2 * (g & 1)]);
+      const float2 v1 = *reinterpret_cast<const float2*>(&r.st[g >> 1][c + 1][2 * (g & 1)]);
+      h[0] = f2_pack(v0.x, v1.x), h[1] = f2_pack(v0.y, v1.y);
     }
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      uint64_t h[2] = {hc[k][0], hc[k][1]};
+      s.h[k][tid] = make_ulonglong2(h[0], h[1]);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const float2 e = *reinterpret_cast<const float2*>(&s.step[4 * k + i][c]);
-        const uint64_t dt = f2_pack(e.x, e.x), dtu = f2_pack(e.x * e.y, e.x * e.y);
-        uint64_t bb[2];
-        ld2<4>(bb, &r.B[4 * k + i][g * 4]);
-#pragma unroll
-        for (int p = 0; p < 2; ++p) h[p] = f2_fma(f2_ex2(f2_mul(dt, a2[p])), h[p], f2_mul(dtu, bb[p]));
+        const ulonglong2 e = s.dt[4 * k + i][cp], bb = *reinterpret_cast<const ulonglong2*>(&s.B[4 * k + i][2 * g]);
+        h[0] = f2_fma(f2_ex2(f2_mul(e.x, a2[0])), h[0], f2_mul(e.y, bb.x));
+        h[1] = f2_fma(f2_ex2(f2_mul(e.x, a2[1])), h[1], f2_mul(e.y, bb.y));
       }
-      hc[k + 1][0] = h[0], hc[k + 1][1] = h[1];
     }
 #pragma unroll 1
     for (int k = 3; k >= 0; --k) {
       uint64_t hs[5][2], av[4][2], bb[4][2];
-#pragma unroll
-      for (int p = 0; p < 2; ++p) hs[0][p] = k == 3 ? hc[3][p] : k == 2 ? hc[2][p] : k == 1 ? hc[1][p] : hc[0][p];
+      hs[0][0] = h[0], hs[0][1] = h[1];
+      if (k > 0) {
+        const ulonglong2 v = s.h[k - 1][tid];
+        h[0] = v.x, h[1] = v.y;
+      }
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const float2 e = *reinterpret_cast<const float2*>(&s.step[4 * k + i][c]);
-        const uint64_t dt = f2_pack(e.x, e.x), dtu = f2_pack(e.x * e.y, e.x * e.y);
-        ld2<4>(bb[i], &r.B[4 * k + i][g * 4]);
+        const ulonglong2 e = s.dt[4 * k + i][cp], v = *reinterpret_cast<const ulonglong2*>(&s.B[4 * k + i][2 * g]);
+        bb[i][0] = v.x, bb[i][1] = v.y;
 #pragma unroll
-        for (int p = 0; p < 2; ++p) {
-          av[i][p] = f2_ex2(f2_mul(dt, a2[p]));
-          hs[i + 1][p] = f2_fma(av[i][p], hs[i][p], f2_mul(dtu, bb[i][p]));
+        for (int n = 0; n < 2; ++n) {
+          av[i][n] = f2_ex2(f2_mul(e.x, a2[n]));
+          hs[i + 1][n] = f2_fma(av[i][n], hs[i][n], f2_mul(e.y, bb[i][n]));
         }
       }
-      float ddt[4], duv[4];
+      uint64_t ddt[4], duv[4];
+      float bc[4];
 #pragma unroll
       for (int i = 3; i >= 0; --i) {
-        const float4 e = s.step[4 * k + i][c];
-        const uint64_t dt = f2_pack(e.x, e.x), gy = f2_pack(e.z, e.z), dtu = f2_pack(e.x * e.y, e.x * e.y);
-        uint64_t cc[2], dd = 0, dv = 0, v[4];
-        ld2<4>(cc, &r.C[4 * k + i][g * 4]);
+        const ulonglong2 e = s.dt[4 * k + i][cp], f = s.gy[4 * k + i][cp];
+        const ulonglong2 cc = *reinterpret_cast<const ulonglong2*>(&s.C[4 * k + i][2 * g]);
+        uint64_t dd = 0, dv = 0;
+        float sum[4];                                          // dB of the two states, dC of them
 #pragma unroll
-        for (int p = 0; p < 2; ++p) {
-          const uint64_t gh = f2_fma(cc[p], gy, cr[p]);        // dL / dh_t
-          cr[p] = f2_mul(gh, av[i][p]);
-          const uint64_t w = f2_mul(cr[p], hs[i][p]);
-          dAa[p] = f2_fma(w, dt, dAa[p]);
-          dd = p == 0 ? f2_mul(w, ar[p]) : f2_fma(w, ar[p], dd);
-          dv = p == 0 ? f2_mul(gh, bb[i][p]) : f2_fma(gh, bb[i][p], dv);
-          v[p] = f2_mul(gh, dtu);
-          v[2 + p] = f2_mul(gy, hs[i + 1][p]);
+        for (int n = 0; n < 2; ++n) {
+          const uint64_t gh = f2_fma(n ? cc.y : cc.x, f.x, cr[n]);        // dL / dh_t
+          cr[n] = f2_mul(gh, av[i][n]);
+          const uint64_t w = f2_mul(cr[n], hs[i][n]);
+          dAa[n] = f2_fma(w, e.x, dAa[n]);
+          dd = n == 0 ? f2_mul(w, ar[n]) : f2_fma(w, ar[n], dd);
+          dv = n == 0 ? f2_mul(gh, bb[i][n]) : f2_fma(gh, bb[i][n], dv);
+          float x, y;
+          f2_unpack(f2_mul(gh, e.y), x, y);
+          sum[n] = x + y;
+          f2_unpack(f2_mul(f.x, hs[i + 1][n]), x, y);
+          sum[2 + n] = x + y;
         }
-        float x, y, x2, y2;
-        f2_unpack(dd, x, y);
-        f2_unpack(dv, x2, y2);
-        duv[i] = (x2 + y2) * e.x;
-        ddt[i] = fmaf(x2 + y2, e.y, x + y);                    // d(dt * B * u) / d dt = B * u
-        // eight sums over the 8 channels of the warp: lane q of them is left with value q (dB of 4 states, dC of 4 states)
-        float f[8];
-#pragma unroll
-        for (int p = 0; p < 4; ++p) f2_unpack(v[p], f[2 * p], f[2 * p + 1]);
-        const bool b4 = lane & 4, b2 = lane & 2, b1 = lane & 1;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const float send = b4 ? f[q] : f[q + 4], keep = b4 ? f[q + 4] : f[q];
-          f[q] = keep + __shfl_xor_sync(0xffffffffu, send, 4);
-        }
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          const float send = b2 ? f[q] : f[q + 2], keep = b2 ? f[q + 2] : f[q];
-          f[q] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
-        }
-        const float send = b1 ? f[0] : f[1], keep = b1 ? f[1] : f[0];
-        s.part[warp][4 * k + i][(b4 ? 16 : 0) + g * 4 + (lane & 3)] = keep + __shfl_xor_sync(0xffffffffu, send, 1);
+        duv[i] = f2_mul(dv, e.x);
+        ddt[i] = f2_fma(dv, f.y, dd);                          // d(dt * B * u) / d dt = B * u
+        // four sums over the 4 lanes of the warp's channels: lane q of them is left with value q
+        const bool b2 = lane & 4, b1 = lane & 1;
+        float p, q;
+        f2_unpack(pair_exchange(f2_pack(sum[0], sum[1]), f2_pack(sum[2], sum[3]), b2, 4), p, q);
+        const float send = b1 ? p : q, keep = b1 ? q : p;
+        bc[i] = keep + __shfl_xor_sync(0xffffffffu, send, 1);
       }
-      const float gd = steps_to_groups<4, CW>(ddt, g), gu = steps_to_groups<4, CW>(duv, g);
-      const int t = 4 * k + g;
-      const float4 e = s.step[t][c];
+      const int t = 4 * k + (g & 3);
+      const ulonglong2 f = s.gy[t][cp];
+      const uint64_t sp = s.sp[t][cp];
+      // sums over the eight groups of states: group i of the lower four is left with d dt of step i, of the upper four with d u
+#pragma unroll
+      for (int i = 0; i < 4; ++i) ddt[i] = pair_exchange(ddt[i], duv[i], g & 4, 16);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) ddt[i] = pair_exchange(ddt[i], ddt[i + 2], g & 2, 8);
+      const uint64_t v = pair_exchange(ddt[0], ddt[1], g & 1, 2);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) s.part[warp][4 * k + i][(lane & 4 ? 16 : 0) + 2 * g + (lane & 1)] = bc[i];
       if (dok && t0 + t < L) {
         const long long off = ((long long)b * L + t0 + t) * Din + d;
-        st(ddelta, off, gd * e.w);
-        du[off] = __float2bfloat16_rn(fmaf(dsk, e.z, gu));
-        dbias = fmaf(gd, e.w, dbias);
-        dDa = fmaf(e.z, e.y, dDa);
+        if (g & 4) {
+          st_pair(&du[off], f2_fma(dsk, f.x, v));
+          acc = f2_fma(f.x, f.y, acc);
+        } else {
+          st_pair(&ddelta[off], f2_mul(v, sp));
+          acc = f2_fma(v, sp, acc);
+        }
       }
     }
     __syncthreads();
 #pragma unroll
-    for (int j = 0; j < SUB * 32 / NT; ++j) {
-      const int i = tid + NT * j, t = i / 32, n = i % 32;
+    for (int j = 0; j < SUB * 8 / NT; ++j) {
+      const int i = tid + NT * j, t = i / 8, n = i % 8 * 4;
       if (t0 + t < L) {
         float* dst = (n < 16 ? dB_part : dC_part) + ((((long long)b * nblk + blockIdx.x / (CB / PC)) * L) + t0 + t) * NS + (n & 15);
-        atomicAdd(dst, s.part[0][t][n] + s.part[1][t][n]);
+        const float4 p = *reinterpret_cast<const float4*>(&s.part[0][t][n]), q = *reinterpret_cast<const float4*>(&s.part[1][t][n]);
+        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(p.x + q.x), "f"(p.y + q.y), "f"(p.z + q.z),
+                     "f"(p.w + q.w) : "memory");
       }
     }
   }
+  float x, y;
 #pragma unroll
-  for (int m = 8; m < 32; m <<= 1) {
-    dDa += __shfl_xor_sync(0xffffffffu, dDa, m);
-    dbias += __shfl_xor_sync(0xffffffffu, dbias, m);
-  }
+  for (int m = 2; m < 16; m <<= 2) acc = f2_add(acc, __shfl_xor_sync(0xffffffffu, acc, m));
   if (dok) {
 #pragma unroll
-    for (int p = 0; p < 2; ++p) {
-      float x, y;
-      f2_unpack(dAa[p], x, y);
-      atomicAdd(&dA[(long long)d * NS + g * 4 + 2 * p], x);
-      atomicAdd(&dA[(long long)d * NS + g * 4 + 2 * p + 1], y);
+    for (int n = 0; n < 2; ++n) {
+      f2_unpack(dAa[n], x, y);
+      atomicAdd(&dA[(long long)d * NS + 2 * g + n], x);
+      atomicAdd(&dA[(long long)(d + 1) * NS + 2 * g + n], y);
     }
-    if (g == 0) {
-      if (dD) atomicAdd(&dD[d], dDa);
-      if (ddelta_bias) atomicAdd(&ddelta_bias[d], dbias);
+    float* sum = g == 0 ? ddelta_bias : g == 4 ? dD : nullptr;
+    if (sum) {
+      f2_unpack(acc, x, y);
+      atomicAdd(&sum[d], x);
+      atomicAdd(&sum[d + 1], y);
     }
   }
 }
@@ -922,7 +1004,7 @@ void s6_scan_bwd(const void* u, const void* delta, bool delta_bf16, const float*
   if (N != NS) throw std::runtime_error("s6_scan: state dimension must be 16");
   if (z && !y_pre) throw std::runtime_error("s6_scan_bwd: the gate's backward needs y_pre");
   dim3 grid(s6_channel_blocks(Din), batch);
-  if (g_bwd_qs == 4 && rows_aligned(Din, {u, delta, Bm, Cm, z, y_pre, dout, state})) {
+  if (g_bwd_qs == 4 && rows_aligned(Din, {u, delta, Bm, Cm, z, y_pre, dout, state, du, ddelta, dB_part, dC_part, dz})) {
     if (delta_bf16)
       launch_bwd_pipe<bf16>(grid, u, delta, delta_bias, softplus, A, Bm, Cm, Dv, z, y_pre, dout, state, du, ddelta, dA,
                             dB_part, dC_part, dD, dz, ddelta_bias, L, Din, st);

@@ -257,3 +257,40 @@ def test_s6_inner_is_convolution_projections_and_scan(bsz, L, c, rank, dtype):
         assert err < 3e-3, (name, err)
     with torch.no_grad():
         assert torch.equal(s6_inner(*a), y)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("din", [16, 1000, 37])          # the pipelined kernels, their last block half full, the general ones
+def test_softplus_of_delta(dtype, din):
+    """dt read off a state checkpoint (no decay, one input) and its derivative off ddelta, against 64 bits, over the range of delta.
+
+    Bound: t = exp(-|x|) has the hardware's 2^-22 and the rounding of its argument, |x| log2(e) 2^-24 ln 2 in t; then 6 roundings."""
+    from ml_experiments_b200.ops.runtime import ops
+
+    x = torch.cat([torch.linspace(-40, 40, din - 9), torch.tensor([0.0, -0.0, 19.99, 20.01, 88.0, -80.0, 100.0, -3e-5, 4e-6])]).to(dtype)
+    length = 20
+    delta = torch.zeros(1, length, din, dtype=dtype)
+    delta[0, 0] = x
+    one = torch.zeros(1, length, 16)
+    one[0, :, 0] = 1.0
+    u = torch.zeros(1, length, din, dtype=torch.bfloat16)
+    u[0, 0] = 1.0
+    delta, u, B, C = (a.cuda() for a in (delta, u, one, one))
+    A = torch.zeros(din, 16, device="cuda")
+    e = lambda *s, t: torch.zeros(*s, device="cuda", dtype=t)
+    y, out = e(1, length, din, t=torch.bfloat16), e(1, length, din, t=torch.bfloat16)
+    state = e(1, 2, 4, din, 4, t=torch.float32)
+    ops().s6_scan_fwd(u, delta, None, True, A, B, C, None, None, y, out, state)
+    dout = torch.zeros_like(u)
+    dout[0, 0] = 1.0
+    ddelta, du, dA = torch.zeros_like(delta), torch.zeros_like(u), torch.zeros_like(A)
+    parts = [e(1, (din + 31) // 32, length, 16, t=torch.float32) for _ in range(2)]
+    ops().s6_scan_bwd(u, delta, None, True, A, B, C, None, None, None, dout, state, du, ddelta, dA, *parts, None, None, None)
+    xd = x.double()
+    dt = torch.where(xd < 0, torch.log1p(torch.exp(xd)), xd + torch.log1p(torch.exp(-xd)))
+    tol = 2.0 ** -22 + 2.0 ** -24 * (xd.abs() * 1.5 + 6)
+    got = state[0, 1, 0, :, 0].double().cpu()
+    assert ((got - dt).abs() <= tol * dt).all()
+    tol = tol + (2.0 ** -8 if dtype == torch.bfloat16 else 0.0)       # (stored as delta's type)
+    sp = 1 / (1 + torch.exp(-xd))
+    assert ((ddelta[0, 0].double().cpu() - sp).abs() <= tol * sp).all()
