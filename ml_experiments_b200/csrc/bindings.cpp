@@ -314,6 +314,35 @@ void axpy_bf16_to_f32(Tensor p, const Tensor& u, const c10::optional<Tensor>& p_
                          (float)alpha, cur_stream());
 }
 
+// p[j] += alpha * its part of u (the tensors' elements one behind the other), with bf16 copies
+void axpy_stack(at::TensorList p, const Tensor& u, at::TensorList p_bf16, double alpha) {
+  TORCH_CHECK(p.size() == p_bf16.size(), "axpy_stack: one bf16 copy per tensor");
+  if (p.empty()) return;
+  const c10::cuda::CUDAGuard guard(u.device());
+  TORCH_CHECK(u.is_cuda() && u.is_contiguous() && u.scalar_type() == at::kBFloat16, "axpy_stack: u contiguous bf16");
+  int64_t total = 0;
+  for (size_t j = 0; j < p.size(); ++j) {
+    TORCH_CHECK(p[j].device() == u.device() && p[j].scalar_type() == at::kFloat && p[j].is_contiguous(), "axpy_stack: p contiguous fp32");
+    TORCH_CHECK(p_bf16[j].device() == u.device() && p_bf16[j].scalar_type() == at::kBFloat16 && p_bf16[j].is_contiguous() &&
+                p_bf16[j].numel() == p[j].numel(), "axpy_stack: copies contiguous bf16, same numel");
+    total += p[j].numel();
+  }
+  TORCH_CHECK(total == u.numel(), "axpy_stack: u has the elements of all tensors");
+  b200::AxpyStack t;
+  t.count = 0;
+  int64_t done = 0;
+  for (size_t j = 0; j < p.size(); ++j) {
+    t.p[t.count] = p[j].data_ptr<float>();
+    t.copy[t.count] = (__nv_bfloat16*)p_bf16[j].data_ptr();
+    t.first[t.count++] = done;
+    done += p[j].numel();
+    t.first[t.count] = done;
+    if (t.count == b200::AXPY_STACK || j + 1 == p.size()) {
+      b200::axpy_stack(t, u.data_ptr(), (float)alpha, cur_stream());
+      t.count = 0;
+    }
+  }
+}
 
 void adam_cautious(Tensor p, const Tensor& g, Tensor m, Tensor v, double b1, double b2, double eps, double step_size, double wd_lr) {
   const c10::cuda::CUDAGuard guard(p.device());
@@ -1180,6 +1209,7 @@ TORCH_LIBRARY(b200, m) {
   m.def("muon_momentum(Tensor g, Tensor(a!) buf, Tensor(b!) out, Tensor(c!) sumsq, float mu, bool nesterov, float grad_scale) -> ()");
   m.def("scale_by_inv_norm(Tensor(a!) x, Tensor sumsq, float eps) -> ()");
   m.def("axpy_bf16_to_f32(Tensor(a!) p, Tensor u, Tensor(b!)? p_bf16, float alpha) -> ()");
+  m.def("axpy_stack(Tensor(a!)[] p, Tensor u, Tensor(b!)[] p_bf16, float alpha) -> ()");
   m.def("comm_signal(int[] peer_flags, int rank, int channel, int epoch, Tensor like) -> ()");
   m.def("adam_shard(int[] grad_ptrs, int[] param_ptrs, int rank, int lo, int hi, int dtype, Tensor(a!) m, Tensor(b!) v, float lr, float beta1, float beta2, float eps, float wd, float bias1, float bias2, Tensor flags, int[] peer_flags, int channel, int epoch, Tensor(c!) status, int max_blocks=0) -> ()");
   m.def("comm_wait(Tensor flags, int world, int channel, int epoch, Tensor(a!) status) -> ()");
@@ -1255,6 +1285,7 @@ TORCH_LIBRARY_IMPL(b200, CUDA, m) {
   m.impl("muon_momentum", &muon_momentum);
   m.impl("scale_by_inv_norm", &scale_by_inv_norm);
   m.impl("axpy_bf16_to_f32", &axpy_bf16_to_f32);
+  m.impl("axpy_stack", &axpy_stack);
   m.impl("comm_signal", &comm_signal);
   m.impl("adam_shard", &adam_shard);
   m.impl("comm_wait", &comm_wait);

@@ -1,6 +1,7 @@
 // Memory-bound fused kernels of the GPT training step (torch-free interface). All tensors are
 // row-major and dense unless a leading dimension is given; "bf16" pointers are __nv_bfloat16.
 #pragma once
+#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <cstdint>
 
@@ -78,6 +79,18 @@ void muon_momentum(const float* g, float* buf, void* out_bf16, float* sumsq, lon
 void scale_by_inv_norm(void* x_bf16, const float* sumsq, long long n, float eps, cudaStream_t s);
 // p (fp32) += alpha * u (bf16) ; optionally also writes the bf16 copy p_bf16 used by the forward GEMMs
 void axpy_bf16_to_f32(float* p, const void* u_bf16, void* p_bf16, long long n, float alpha, cudaStream_t s);
+// The same for up to AXPY_STACK tensors in one launch: tensor j takes elements [first[j], first[j + 1]) of u. `block` and `vec` are filled
+// in by the call.
+constexpr int AXPY_STACK = 64;
+struct AxpyStack {
+  float* p[AXPY_STACK];
+  __nv_bfloat16* copy[AXPY_STACK];      // or null
+  long long first[AXPY_STACK + 1];
+  int block[AXPY_STACK];
+  unsigned long long vec;
+  int count;
+};
+void axpy_stack(AxpyStack& t, const void* u_bf16, float alpha, cudaStream_t s);
 
 // ---- RMS norm + rotary of the current speedrun GPT (norm_rope.cu): x [batch, T, H, D] bf16 with element strides st
 // (between tokens; batch entries are T * st apart) and sh (between heads), tables [T_max, tab_w] bf16 (tab_w = D, or 2 D

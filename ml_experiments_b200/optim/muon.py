@@ -137,6 +137,14 @@ class Muon(torch.optim.Optimizer):
         else:
             u = newton_schulz_(ent["stack"], coeffs, self._work)
         alpha = -lr * max(1.0, r / c) ** 0.5
+        if all(p.dtype == torch.float32 for p, _ in plist):       # one launch for the stack, with the bf16 copies
+            shadows = [get_shadow_buffer(p, torch.bfloat16) for p, _ in plist]
+            shadows = [torch.empty(p.shape, dtype=torch.bfloat16, device=p.device) if sh is None else sh for sh, (p, _) in zip(shadows, plist)]
+            o.axpy_stack([p for p, _ in plist], u, shadows, alpha)
+            for (p, _), sh in zip(plist, shadows):
+                mark_modified(p)
+                set_shadow(p, sh)
+            return
         slot = 0
         for p, nmat in plist:
             upd = u[slot:slot + nmat].view(p.shape)

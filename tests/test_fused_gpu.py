@@ -391,6 +391,22 @@ def test_axpy_tails_and_alignment(n, off):
     assert bool((copy[:off] == 7.0).all())
 
 
+@pytest.mark.parametrize("sizes", [[1], [2048 * 8 + 5, 0, 7, 8, 9], [333, 256] * 32, [8 * 300] * 65 + [1, 3]])
+def test_axpy_stack_is_axpy_of_each(sizes):
+    """One tensor, empty ones, parts of u that start off the 16-byte boundary, a full table of 64 and more than that."""
+    from ml_experiments_b200.ops.runtime import ops
+
+    g = torch.Generator(device="cuda").manual_seed(len(sizes))
+    ps = [torch.randn(n, generator=g, device="cuda") for n in sizes]
+    u = torch.randn(sum(sizes), generator=g, device="cuda").bfloat16()
+    want = [torch.addcmul(p.double(), v.double(), torch.full_like(v, -0.25).double()).float() for p, v in zip(ps, u.split(sizes))]
+    copies = [torch.full((n,), 7.0, device="cuda", dtype=torch.bfloat16) for n in sizes]
+    ops().axpy_stack(ps, u, copies, -0.25)
+    assert all(torch.equal(p, w) and torch.equal(c, w.bfloat16()) for p, w, c in zip(ps, want, copies))
+    with pytest.raises(RuntimeError, match="elements of all"):
+        ops().axpy_stack(ps, u.repeat(2), copies, -0.25)
+
+
 @pytest.mark.parametrize("elems", [8, 4096 + 8, 10, 2 * 333])
 def test_stack_scale_vector_and_pair_paths(elems):
     from ml_experiments_b200.ops.runtime import ops
