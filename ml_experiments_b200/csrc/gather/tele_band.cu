@@ -7,11 +7,11 @@
 //   forward   Y  = W X            queries stay, the block walks the keys of its band
 //   rows      S  = dY Xᵀ, read at the taps: gradients of stride, phase, table and exponent; queries stay
 //   dX        dX = Wᵀ dY          keys stay, the block walks the query tiles that reach them: nothing is added in memory
-// 8 x 16384 tokens x 4 heads of 64, 235 taps: forward 0.97 ms (3.57 gathered), rows 1.35 + dX 1.75 (10.3 gathered). The bound is the
+// 8 x 16384 tokens x 4 heads of 64, 235 taps: forward 1.12 ms (3.57 gathered), rows 1.35 + dX 2.0 (10.3 gathered). The bound is the
 // issue of the tap formulas and of the conversion of tiles (54 to 62 % of the issue slots; the tensor pipe is 15 % busy).
 //
-// Weights are evaluated in fp32 and enter the product as a sum of bf16 terms (two: 16 bits of mantissa, where the result is
-// rounded to bf16; three: all 24, where the gradient is wanted in fp32); x and dY are bf16 already, sums are fp32.
+// Weights are evaluated in fp32 and enter the product as a sum of three bf16 terms, which hold all 24 bits of them; x and dY are
+// bf16 already, sums are fp32. (With two terms, 16 bits: 0.97 and 1.75 ms.)
 // A thread builds 32 keys of one query in a column of shared memory of its own ([cell][thread]: whatever cells the lanes of a
 // warp touch, they are in 32 different banks), then splits them into terms. The queries of a tile are sorted by stride, so the lanes
 // of a warp have about the same number of taps in a step.
@@ -36,6 +36,7 @@ constexpr int ROWS = 128;             // queries of a block (forward, rows) / ke
 constexpr int STEP = 64;              // keys (dX: queries) of a step
 constexpr int SEG = 32;               // keys that a thread builds in a step
 constexpr int BUILDERS = 256;
+constexpr int TERMS = 3;              // bf16 terms of a weight
 constexpr int THREADS = BUILDERS + 64;   // two warps more: one issues the MMAs, one the TMA loads
 // A tap of keys c - 1, c is written at cells c + 1, c + 2: cells 0, 1 and SEG + 2 are for what belongs to other segments
 constexpr int CELL_BYTES = (SEG + 3) * BUILDERS * 4;
@@ -290,9 +291,9 @@ __device__ __forceinline__ void fill_weights(const BP& p, float* wt, float* tab,
 template <int N>
 struct FwdShape {
   static constexpr int NS = N / 64, XST = N == 128 ? 1 : 2;
-  static constexpr int NAB = N == 128 ? 2 : 3;     // tiles of W in tensor memory
+  static constexpr int NAB = N == 128 ? 1 : 2;     // tiles of W in tensor memory, of which two blocks share the 512 columns
   static constexpr int X_BYTES = NS * STEP * 128;
-  static constexpr uint32_t COLS = 256;            // N of results, the tiles in two terms of 32
+  static constexpr uint32_t COLS = 256;            // N of results, the tiles in three terms of 32
   static size_t smem(int half) { return (size_t)XST * X_BYTES + CELL_BYTES + (size_t)(half + 2) * ROWS * 4 + 1024; }
 };
 
@@ -311,11 +312,12 @@ __device__ __noinline__ float gathered(const Taps& t, const float* wt, const bf1
 }
 
 template <int N>
-__global__ void __launch_bounds__(THREADS, N == 64 ? 2 : 1)
+__global__ void __launch_bounds__(THREADS, 2)
 tele_band_fwd_kernel(const __grid_constant__ CUtensorMap tmX, const BP p) {
   using F = FwdShape<N>;
   constexpr int XST = F::XST, NAB = F::NAB, NBAR = 2 * NAB + 1 + 2 * XST;
-  constexpr uint32_t A_COL = N, TERM = 32, BUF = 64;
+  constexpr uint32_t A_COL = N, TERM = 32, BUF = TERMS * TERM;
+  static_assert(A_COL + NAB * BUF <= F::COLS, "tensor memory");
   extern __shared__ __align__(1024) uint8_t raw[];
   // (rounded up by an offset: through an integer the compiler would lose sight of the address space and use generic accesses)
   uint8_t* sX = raw + (-smem_u32(raw) & 1023u);
@@ -365,7 +367,7 @@ tele_band_fwd_kernel(const __grid_constant__ CUtensorMap tmX, const BP p) {
       tc_fence_after_sync();
       if (elect_one_sync()) {
 #pragma unroll
-        for (int term = 0; term < 2; ++term)
+        for (int term = 0; term < TERMS; ++term)
 #pragma unroll
           for (int ks = 0; ks < STEP / 16; ++ks)
             tc_mma_f16_ts(fr.tmem, fr.tmem + A_COL + bf * BUF + term * TERM + ks * 8, xd + (st * F::X_BYTES + ks * 2048) / 16, idesc,
@@ -397,7 +399,7 @@ tele_band_fwd_kernel(const __grid_constant__ CUtensorMap tmX, const BP p) {
       if (__any_sync(0xffffffffu, *abort_flag)) break;
       tc_fence_after_sync();
       if (any || !(zero >> bf & 1)) {
-        uint32_t hi[16], lo[16];
+        uint32_t o[TERMS][16];
 #pragma unroll
         for (int k = 0; k < 16; ++k) {
           float v0 = 0.f, v1 = 0.f;
@@ -406,12 +408,12 @@ tele_band_fwd_kernel(const __grid_constant__ CUtensorMap tmX, const BP p) {
             v0 = c[0], v1 = c[BUILDERS];
             c[0] = 0.f, c[BUILDERS] = 0.f;
           }
-          hi[k] = take_term(v0, v1);
-          lo[k] = pack_bf16x2(v0, v1);
+#pragma unroll
+          for (int term = 0; term < TERMS; ++term) o[term][k] = take_term(v0, v1);
         }
         const uint32_t at = fr.tmem + lane_off + A_COL + bf * BUF + part * 16;
-        tmem_st_32x32b_x16(at, hi);
-        tmem_st_32x32b_x16(at + TERM, lo);
+#pragma unroll
+        for (int term = 0; term < TERMS; ++term) tmem_st_32x32b_x16(at + term * TERM, o[term]);
         tmem_st_wait();
         zero = any ? zero & ~(1u << bf) : zero | (1u << bf);
       }
@@ -706,14 +708,18 @@ tele_band_plan_kernel(const float* __restrict__ freq, const float* __restrict__ 
   if (i == 0) ranges[blockIdx.x] = make_int2(min(wlo[0], wlo[1]), max(whi[0], whi[1]));
 }
 
-template <int N, int NT>
+template <int N>
 struct DxShape {
   static constexpr int NS = N / 64;
   static constexpr int A_BYTES = 2 * STEP * 128, Q_BYTES = NS * STEP * 128;    // one term of Wᵀ: 64 queries x 128 keys
   static constexpr uint32_t COLS = N;
-  // one stage of dY suffices where two would keep a second block off the multiprocessor
-  static int stages(int K) { return N == 64 && K <= 32 ? 2 : 1; }
-  static size_t smem(int K) { return (size_t)NT * A_BYTES + stages(K) * Q_BYTES + CELL_BYTES + 2 * (size_t)(K + 1) * STEP * 4 + 1024; }
+  // Two blocks share a multiprocessor, which takes K up to 64 (N = 128: 43). One copy of the tables (a barrier a step more) or one stage of
+  // dY is enough where the second would keep the other block off.
+  static constexpr int ROOM = (233472 - 2 * 1024) / 2 - 2048 - 1024 - TERMS * A_BYTES - CELL_BYTES;   // for the two, beside the static part
+  static __host__ __device__ bool fits(int stages, int tables, int K) { return stages * Q_BYTES + tables * (K + 1) * STEP * 4 <= ROOM; }
+  static __host__ __device__ int stages(int K) { return fits(2, 2, K) ? 2 : 1; }
+  static __host__ __device__ int tables(int K) { return !fits(1, 2, K) && fits(1, 1, K) ? 1 : 2; }
+  static size_t smem(int K) { return (size_t)TERMS * A_BYTES + stages(K) * Q_BYTES + CELL_BYTES + tables(K) * (size_t)(K + 1) * STEP * 4 + 1024; }
 };
 
 // As `gathered`, for a gradient: only the queries that sample this key count.
@@ -744,15 +750,15 @@ __device__ __noinline__ float gathered_dx(const BP& p, int b, int h, int key, co
 
 constexpr int MAX_TILES = 512;       // query tiles of a sequence: 32768 tokens
 
-template <int N, int NT>
-__global__ void __launch_bounds__(THREADS, N == 64 && NT == 2 ? 2 : 1)
+template <int N, typename TO>
+__global__ void __launch_bounds__(THREADS, 2)
 tele_band_dx_kernel(const __grid_constant__ CUtensorMap tmG, const BP p) {
-  using F = DxShape<N, NT>;
+  using F = DxShape<N>;
   constexpr int NBAR = 7;
   extern __shared__ __align__(1024) uint8_t raw[];
   uint8_t* sA = raw + (-smem_u32(raw) & 1023u);
-  uint8_t* sG = sA + NT * F::A_BYTES;
-  const int GST = N == 64 && p.K <= 32 ? 2 : 1;
+  uint8_t* sG = sA + TERMS * F::A_BYTES;
+  const int GST = F::stages(p.K), TABS = F::tables(p.K);
   float* cells = reinterpret_cast<float*>(sG + GST * F::Q_BYTES);
   float* tabs = cells + CELL_BYTES / 4;
   __shared__ uint64_t bars[NBAR];
@@ -811,7 +817,7 @@ tele_band_dx_kernel(const __grid_constant__ CUtensorMap tmG, const BP p) {
       tc_fence_after_sync();
       if (elect_one_sync()) {
 #pragma unroll
-        for (int term = 0; term < NT; ++term)
+        for (int term = 0; term < TERMS; ++term)
 #pragma unroll
           for (int ks = 0; ks < STEP / 16; ++ks)
             tc_mma_f16(fr.tmem, ad + (term * F::A_BYTES + ks * 2048) / 16, gd + (st * F::Q_BYTES + ks * 2048) / 16, idesc, (i | term | ks) != 0);
@@ -846,7 +852,8 @@ tele_band_dx_kernel(const __grid_constant__ CUtensorMap tmG, const BP p) {
       const int bits = __float_as_int(rec.b.w), q = bits & 255, l = list[i] * STEP + q;
       const bool ok = l < p.L;
       const float expo = rec.b.z;
-      float* tab = tabs + (i & 1) * (p.K + 1) * STEP;
+      float* tab = tabs + (TABS == 2 ? i & 1 : 0) * (p.K + 1) * STEP;
+      if (TABS == 1 && i > 0) builders_sync<BUILDERS>();   // nobody reads the last one any more
       const float* krow = p.kern + (((long long)b * p.L + (ok ? l : 0)) * p.H + h) * p.K;
       if (small) {
         float* to = tab + 4 * seg * STEP + slot_q;
@@ -872,7 +879,7 @@ tele_band_dx_kernel(const __grid_constant__ CUtensorMap tmG, const BP p) {
       uint8_t* dst = sA + (seg >> 1) * (STEP * 128) + q * 128;
 #pragma unroll
       for (int ch = 0; ch < 4; ++ch) {
-        uint32_t o[NT][4];
+        uint32_t o[TERMS][4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           float v0 = 0.f, v1 = 0.f;
@@ -882,11 +889,11 @@ tele_band_dx_kernel(const __grid_constant__ CUtensorMap tmG, const BP p) {
             c[0] = 0.f, c[BUILDERS] = 0.f;
           }
 #pragma unroll
-          for (int term = 0; term < NT; ++term) o[term][k] = take_term(v0, v1);
+          for (int term = 0; term < TERMS; ++term) o[term][k] = take_term(v0, v1);
         }
         const int at = (((seg & 1) * 4 + ch) ^ (q & 7)) * 16;
 #pragma unroll
-        for (int term = 0; term < NT; ++term)
+        for (int term = 0; term < TERMS; ++term)
           *reinterpret_cast<uint4*>(dst + term * F::A_BYTES + at) = make_uint4(o[term][0], o[term][1], o[term][2], o[term][3]);
       }
       fence_proxy_async_smem();
@@ -910,7 +917,7 @@ tele_band_dx_kernel(const __grid_constant__ CUtensorMap tmG, const BP p) {
           o[k] = n > 0 ? __uint_as_float(v[k]) : 0.f;
           if (!(fabsf(o[k]) <= FLT_MAX)) o[k] = gathered_dx(p, b, h, key, list, n, c0 + k);
         }
-        if (NT == 2) {
+        if (sizeof(TO) == 2) {
           uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(p.dx) + at + c0);
 #pragma unroll
           for (int k = 0; k < 2; ++k)
@@ -947,10 +954,10 @@ void configure() {
   opt_in(tele_band_fwd_kernel<128>);
   opt_in(tele_band_rows_kernel<64>);
   opt_in(tele_band_rows_kernel<128>);
-  opt_in(tele_band_dx_kernel<64, 2>);
-  opt_in(tele_band_dx_kernel<64, 3>);
-  opt_in(tele_band_dx_kernel<128, 2>);
-  opt_in(tele_band_dx_kernel<128, 3>);
+  opt_in(tele_band_dx_kernel<64, bf16>);
+  opt_in(tele_band_dx_kernel<64, float>);
+  opt_in(tele_band_dx_kernel<128, bf16>);
+  opt_in(tele_band_dx_kernel<128, float>);
   cfg.done(dev);
 }
 BP params(const void* x, const float* freq, const float* phase, const float* kern, const float* expo, int L, int H, int D, int K, int half,
@@ -1020,10 +1027,10 @@ void tele_band_bwd(const void* x, const float* freq, const float* phase, const f
   if (D == 128) tele_band_rows_kernel<128><<<grid, RTHREADS, RowsShape<128>::smem(half), s>>>(tx, p);
   else tele_band_rows_kernel<64><<<grid, RTHREADS, RowsShape<64>::smem(half), s>>>(tx, p);
   chk("tele_band_rows");
-  if (D == 128 && dx_f32) tele_band_dx_kernel<128, 3><<<grid, THREADS, DxShape<128, 3>::smem(K), s>>>(tg, p);
-  else if (D == 128) tele_band_dx_kernel<128, 2><<<grid, THREADS, DxShape<128, 2>::smem(K), s>>>(tg, p);
-  else if (dx_f32) tele_band_dx_kernel<64, 3><<<grid, THREADS, DxShape<64, 3>::smem(K), s>>>(tg, p);
-  else tele_band_dx_kernel<64, 2><<<grid, THREADS, DxShape<64, 2>::smem(K), s>>>(tg, p);
+  if (D == 128 && dx_f32) tele_band_dx_kernel<128, float><<<grid, THREADS, DxShape<128>::smem(K), s>>>(tg, p);
+  else if (D == 128) tele_band_dx_kernel<128, bf16><<<grid, THREADS, DxShape<128>::smem(K), s>>>(tg, p);
+  else if (dx_f32) tele_band_dx_kernel<64, float><<<grid, THREADS, DxShape<64>::smem(K), s>>>(tg, p);
+  else tele_band_dx_kernel<64, bf16><<<grid, THREADS, DxShape<64>::smem(K), s>>>(tg, p);
   chk("tele_band_dx");
 }
 

@@ -67,6 +67,29 @@ def test_telephone_band(B, L, H, D, K, half, freq, dtype):
         assert _rel(a.grad, b.grad) < tol, (name, _rel(a.grad, b.grad), tol)
 
 
+@pytest.mark.parametrize("D,H", [(16, 4), (64, 2), (128, 2)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_telephone_band_weights_have_24_bits(D, H, dtype):
+    """Two rows of opposite sign and nothing else: a result is the difference of the weights of two neighbouring taps, 6.8e-5 of them. It is
+    off by their rounding to fp32 (three of 2^-24 each, 0.3 % of it) and by its own to bf16 (0.2 %); by 16 bits it would be off by 10 %."""
+    from ml_experiments_b200.ops import fused_taps as T
+
+    L, K, half, j = 1000, 16, 54, 500
+    pair = torch.zeros(1, L, H * D, device="cuda", dtype=dtype)
+    pair[:, j], pair[:, j + 1] = 1, -1
+    x = pair.clone().requires_grad_()
+    one, zero = torch.ones(1, L, H, device="cuda"), torch.zeros(1, L, H, device="cuda")
+    kern = (1 + torch.arange(K, device="cuda") / 256).expand(1, L, H, K).contiguous()
+    y = T.telephone_gather(x, one, zero, kern, torch.zeros(1, L, 1, device="cuda"), H, half, half * 16.0)
+    y.backward(pair)
+    tap = (torch.arange(L, device="cuda") - j).abs().double()
+    step = (K - 1) / (half * 16.0) / 256
+    want = step * torch.where(torch.arange(L, device="cuda") <= j, -1.0, 1.0).double()
+    both = (tap <= half) & ((torch.arange(L, device="cuda") - j - 1).abs() <= half)
+    for got in (y, x.grad):                     # (the gradient is the same sum over the queries that sample a row)
+        assert ((got[0, both].double() - want[both, None]).abs() / step).max().item() < 1e-2
+
+
 def test_telephone_band_keeps_what_is_not_finite_where_it_is_sampled():
     """A row of x (of the gradient) that is not finite reaches the queries that sample it (the rows that it samples) and no others,
     although products with weights of zero are formed."""
