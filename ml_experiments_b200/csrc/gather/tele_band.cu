@@ -613,20 +613,23 @@ tele_band_rows_kernel(const __grid_constant__ CUtensorMap tmX, const BP p) {
       float* dk = tab + p.K * ROWS * (1 + part) + row;
       float a = 0.f, c = 0.f;                              // of the last tap's entry and the next (entries never fall)
       int last = -2;
-      for (int s = part; s <= p.half; s += 4) {
-        float dw[2];
+      // a tap outside the sequence counts for nothing, whatever its formulas would give (a stride may be infinite, or no number)
+      const int most = t.lo <= t.hi ? p.half : -1;
+      for (int s = part; s <= most; s += 4) {
+        float dw[2], ar[2];
         Entry e[2];
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
           const int u = min(s + 2 * j, p.half);
           const bool in = s + 2 * j <= p.half && ((u >= t.lo && u <= t.hi) || (-u >= t.lo && -u <= t.hi));
+          ar[j] = in ? (float)u * t.f : 0.f;
           e[j] = table_entry(tab + row, ROWS, p.K, (float)u * t.f * p.inv_rec);
           dw[j] = in ? sums[u * ROWS + row] : 0.f;
           if (!in) e[j].v = e[j].slope = 0.f;
         }
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
-          const float ar = (float)(s + 2 * j) * t.f, base = 1.f + ar * p.invL, lg = log2f(base);
+          const float base = 1.f + ar[j] * p.invL, lg = log2f(base);
           const float dkv = dw[j] * exp2f(-expo * lg), dv = dkv * e[j].v;
           a = (e[j].lo == last ? a : e[j].lo == last + 1 ? c : 0.f) + dkv * (1.f - e[j].wh);
           c = (e[j].lo == last ? c : 0.f) + dkv * e[j].wh;

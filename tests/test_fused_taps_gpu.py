@@ -113,6 +113,31 @@ def test_telephone_band_keeps_what_is_not_finite_where_it_is_sampled():
     assert bad.any() and torch.equal(leaves[0].grad[:, inner].isfinite().logical_not(), bad)
 
 
+@pytest.mark.parametrize("D", [32, 128])
+@pytest.mark.parametrize("stride", [float("nan"), float("inf"), float("-inf"), 1e38, -1e38])
+def test_telephone_band_strides_that_leave_the_sequence(D, stride):
+    """A stride that is no number or infinite has no tap in the sequence (0 * stride is no number either): nothing comes out of it, and its
+    gradients are zero. A very large one has tap 0 alone, as 1e6 has."""
+    from ml_experiments_b200.ops import fused_taps as T
+
+    B, L, H, half, at = 1, 700, 2, 54, (0, slice(100, 700, 150), 0)
+    ins, dout = _band_inputs(B, L, H, D, 16, 6, "wide")
+    ins[4][0, ::100] *= -1                       # weights that grow with the distance
+    grads, ys = [], []
+    for f in (stride, 1e6):
+        ins[1][at] = f
+        leaves = [t.clone().requires_grad_(True) for t in ins]
+        ys.append(T.telephone_gather(*leaves, H, half, half * 16.0))
+        ys[-1].backward(dout)
+        grads.append([t.grad for t in leaves])
+        assert all(t.isfinite().all() for t in [ys[-1], *grads[-1]])
+    if abs(stride) < float("inf"):
+        assert torch.equal(*ys) and all(torch.equal(a, b) for a, b in zip(*grads))
+        assert all(g[at].abs().sum() > 0 for g in grads[0][2:4])
+    else:
+        assert not ys[0].view(B, L, H, D)[at].any() and not any(g[at].any() for g in grads[0][1:4])
+
+
 @pytest.mark.parametrize("B,L,H,D,K,half", [(2, 300, 4, 64, 64, 29), (1, 1000, 2, 16, 16, 9), (2, 130, 3, 128, 8, 3), (1, 257, 8, 8, 64, 12)])
 def test_adaptive_local_fused(B, L, H, D, K, half):
     from ml_experiments_b200.ops import fused_taps as T
