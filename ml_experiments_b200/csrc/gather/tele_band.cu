@@ -64,6 +64,33 @@ struct BP {
 
 template <int N>
 __device__ __forceinline__ void builders_sync() { asm volatile("bar.sync 1, %0;" ::"n"(N) : "memory"); }
+template <int N>
+__device__ __forceinline__ bool builders_any(bool v) {
+  int any;
+  asm volatile("{\n.reg .pred p, q;\nsetp.ne.b32 p, %1, 0;\nbar.red.or.pred q, 1, %2, p;\nselp.b32 %0, 1, 0, q;\n}\n" : "=r"(any) : "r"((int)v), "n"(N) : "memory");
+  return any != 0;
+}
+__device__ __forceinline__ bool is_finite(float v) { return fabsf(v) <= FLT_MAX; }
+// The columns of `of` that are no number
+__device__ __forceinline__ uint32_t nan_columns(const float (&of)[16]) {
+  uint32_t m = 0;
+#pragma unroll
+  for (int k = 0; k < 16; ++k) m |= of[k] == of[k] ? 0u : 1u << k;
+  return m;
+}
+// 16 columns of a row, times a weight
+__device__ __forceinline__ void add_row(float (&acc)[16], float w, const uint4* row) {
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const uint4 u = row[i];
+    const uint32_t v[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      acc[8 * i + 2 * k] = fmaf(w, __uint_as_float(v[k] << 16), acc[8 * i + 2 * k]);
+      acc[8 * i + 2 * k + 1] = fmaf(w, __uint_as_float(v[k] & 0xffff0000u), acc[8 * i + 2 * k + 1]);
+    }
+  }
+}
 
 // The taps of one query. A position is rounded three times, as the operator states it, (l + tap * stride) + phase: which rows are read is
 // part of its definition. Positions never fall along the taps; the sign of the stride only swaps the taps' names.
@@ -297,18 +324,21 @@ struct FwdShape {
   static size_t smem(int half) { return (size_t)XST * X_BYTES + CELL_BYTES + (size_t)(half + 2) * ROWS * 4 + 1024; }
 };
 
-// A result that is not finite: a row of x that the query does not sample may have spoiled it, as 0 * inf does. Tap by tap, then.
-__device__ __noinline__ float gathered(const Taps& t, const float* wt, const bf16* xcol, long long rs, int L) {
-  float acc = 0.f;
-  for (int s = t.lo; s <= t.hi; ++s) {
+// Results that are not finite: a row of x that the query does not sample may have spoiled them, as 0 * inf does. Tap by tap, then, 16 columns
+// at a time, until all that are wanted are no numbers, which they then stay. 8 x 16384 x 4 heads of 64: 1.18 ms where all of x is NaN, 7.1
+// with some NaN in every 64th row (3.6 in the gather, whatever the values).
+__device__ __noinline__ void gathered(const Taps& t, const float* wt, const bf16* xcol, long long rs, int L, uint32_t wanted, float (&acc)[16]) {
+#pragma unroll
+  for (int k = 0; k < 16; ++k) acc[k] = 0.f;
+  for (int s = t.lo; s <= t.hi && (wanted & ~nan_columns(acc)); ++s) {
     const float w = wt[(s < 0 ? -s : s) * ROWS];
     if (w == 0.f) continue;
     const float pos = fminf(tap_position(t, (float)s), last_position(L));
     const int fl = floor_int(pos);
     const float fr = pos - (float)fl;
-    acc += w * (1.f - fr) * __bfloat162float(xcol[fl * rs]) + w * fr * __bfloat162float(xcol[(fl + 1) * rs]);
+    add_row(acc, w * (1.f - fr), reinterpret_cast<const uint4*>(xcol + fl * rs));
+    add_row(acc, w * fr, reinterpret_cast<const uint4*>(xcol + (fl + 1) * rs));
   }
-  return acc;
 }
 
 template <int N>
@@ -431,14 +461,23 @@ tele_band_fwd_kernel(const __grid_constant__ CUtensorMap tmX, const BP p) {
       tmem_ld_32x32b_x16(fr.tmem + lane_off + c0, v);
       tmem_ld_wait();
       if (ok) {
+        float y[16];
+        uint32_t bad = 0;
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+          y[k] = band.n > 0 ? __uint_as_float(v[k]) : 0.f;
+          bad |= is_finite(y[k]) ? 0u : 1u << k;
+        }
+        if (bad) {
+          float g[16];
+          gathered(t, wrow, xcol + c0, (long long)p.H * p.D, p.L, bad, g);
+#pragma unroll
+          for (int k = 0; k < 16; ++k)
+            if (bad >> k & 1) y[k] = g[k];
+        }
         uint32_t o[8];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          float a = band.n > 0 ? __uint_as_float(v[2 * k]) : 0.f, c = band.n > 0 ? __uint_as_float(v[2 * k + 1]) : 0.f;
-          if (!(fabsf(a) <= FLT_MAX)) a = gathered(t, wrow, xcol + c0 + 2 * k, (long long)p.H * p.D, p.L);
-          if (!(fabsf(c) <= FLT_MAX)) c = gathered(t, wrow, xcol + c0 + 2 * k + 1, (long long)p.H * p.D, p.L);
-          o[k] = pack_bf16x2(a, c);
-        }
+        for (int k = 0; k < 8; ++k) o[k] = pack_bf16x2(y[2 * k], y[2 * k + 1]);
         reinterpret_cast<uint4*>(orow + c0)[0] = make_uint4(o[0], o[1], o[2], o[3]);
         reinterpret_cast<uint4*>(orow + c0)[1] = make_uint4(o[4], o[5], o[6], o[7]);
       }
@@ -725,30 +764,66 @@ struct DxShape {
   static size_t smem(int K) { return (size_t)TERMS * A_BYTES + stages(K) * Q_BYTES + CELL_BYTES + tables(K) * (size_t)(K + 1) * STEP * 4 + 1024; }
 };
 
-// As `gathered`, for a gradient: only the queries that sample this key count.
-__device__ __noinline__ float gathered_dx(const BP& p, int b, int h, int key, const uint16_t* list, int n, int c) {
-  float acc = 0.f;
-  for (int i = 0; i < n; ++i) {
-    for (int l = list[i] * STEP; l < min(list[i] * STEP + STEP, p.L); ++l) {
-      const long long bl = (long long)b * p.L + l, row = bl * p.H + h;
-      const float f = fabsf(p.freq[row]), ph = p.phase[row];
-      const int2 in = inside(f, ph, l, p.L, p.half);
-      const Taps t = make_taps(f, ph, l, in.x, in.y, p.L);
-      const int2 r = tap_range(t, key, key + 1, p.L);
-      const float g = __bfloat162float(p.dout[row * p.D + c]);
-      for (int s = r.x; s <= r.y; ++s) {
-        const float pos = fminf(tap_position(t, (float)s), last_position(p.L));
-        const int fl = floor_int(pos);
-        const float fr = pos - (float)fl;
-        const float ar = (float)abs(s) * f;
-        const float w = table_entry(p.kern + row * p.K, 1, p.K, ar * p.inv_rec).v * decay(p.expo[bl], ar, p.invL);
-        if (w == 0.f) continue;
-        if (fl == key) acc += w * (1.f - fr) * g;
-        if (fl + 1 == key && fr != 0.f) acc += w * fr * g;
-      }
+// Weights of a query's taps by the formula, from its table's values at trow[k * STEP] (entry K is met with weight zero only)
+struct TapWeights {
+  const float* trow;
+  float expo, step_entry, step_base, last_entry;
+  __device__ __forceinline__ void operator()(int s, float (&w)[2]) const {
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const float as = (float)abs(s + j), idx = fminf(as * step_entry, last_entry), m = floor_magic(idx);
+      const float* e = trow + (__float_as_int(m) - MAGIC_BITS) * STEP;
+      w[j] = fmaf(idx - (m - MAGIC), e[STEP] - e[0], e[0]) * exp2f(-expo * log2f(fmaf(as, step_base, 1.f)));
     }
   }
-  return acc;
+};
+__device__ __forceinline__ TapWeights tap_weights(const BP& p, const float* trow, float expo, float f) {
+  return TapWeights{trow, expo, f * p.inv_rec * (float)(p.K - 1), f * p.invL, (float)(p.K - 1)};
+}
+__device__ __forceinline__ Taps plan_taps(const float4& a, const float4& b, int kmin, int kmax, int l) {
+  const int bits = __float_as_int(b.w);
+  return Taps{a.x, a.y, a.z, a.w, b.x, b.y, l, ((bits >> 8) & 0xfff) - 512, (bits >> 20) - 512, kmin, kmax};
+}
+
+// As `gathered`, for a gradient: only the queries that sample this thread's key count. All builders together, tile by tile: the weights are
+// formed as for the product, and read where they are not zero. cells: all zero, before and after; rows: 4 KB for 16 columns of the tile's
+// dY, from c0 for the first half of the threads and from c0 + next for the others (none from D on). 8 x 16384 x 4 heads of 64, whole backward:
+// 5.4 ms where all of dY is NaN, 31 with some NaN in every 64th row (10.3 in the gather; a thread with its own element's taps: 87).
+__device__ __noinline__ void gathered_dx(const BP& p, int b, int h, int k0, const uint16_t* list, int n, long long plan, float* cells, float* tab, uint4* rows,
+                                         int c0, int next, uint32_t wanted, float (&acc)[16]) {
+  const int tid = threadIdx.x, slot_q = tid & (STEP - 1), seg = tid / STEP;
+  float* col = cells + tid;
+  const float* mine = cells + ((tid & 31) + 2) * BUILDERS + (tid & (ROWS - 1)) / SEG * STEP;     // this key's cells of the tile's queries
+  const int half_row = (tid & 3) >> 1, c = c0 + half_row * next + (tid & 1) * 8;                 // what this thread copies
+  const uint4* row = rows + tid / ROWS * 2;
+#pragma unroll
+  for (int k = 0; k < 16; ++k) acc[k] = 0.f;
+  for (int i = 0; i < n && builders_any<BUILDERS>((wanted & ~nan_columns(acc)) != 0); ++i) {
+    const Query* queries = p.queries + (plan + list[i]) * STEP;
+    const float4 qa = queries[slot_q].a, qb = queries[slot_q].b;
+    const int l = list[i] * STEP + (__float_as_int(qb.w) & 255);
+    const bool ok = l < p.L;
+    stage_table(tab, p.kern + (((long long)b * p.L + (ok ? l : 0)) * p.H + h) * p.K, ok, slot_q, STEP, seg, 4, p.K, p.kvec);
+    if (seg == 3) tab[p.K * STEP + slot_q] = 0.f;
+    const int lc = list[i] * STEP + (__float_as_int(queries[tid >> 2].b.w) & 255);
+    rows[tid] = lc < p.L && c < p.D ? *reinterpret_cast<const uint4*>(p.dout + (((long long)b * p.L + lc) * p.H + h) * p.D + c) : make_uint4(0, 0, 0, 0);
+    builders_sync<BUILDERS>();
+    const bool any = add_taps(col, plan_taps(qa, qb, queries[slot_q].kmin, queries[slot_q].kmax, l), k0 + seg * SEG, p.L,
+                              tap_weights(p, tab + slot_q, qb.z, qa.x));
+    builders_sync<BUILDERS>();
+    if (wanted) {
+#pragma unroll 4
+      for (int q = 0; q < STEP; ++q) {
+        const float w = mine[q];
+        if (w != 0.f) add_row(acc, w, row + q * 4);
+      }
+    }
+    builders_sync<BUILDERS>();
+    if (any) {
+#pragma unroll
+      for (int k = 2; k < SEG + 2; ++k) col[k * BUILDERS] = 0.f;
+    }
+  }
 }
 
 constexpr int MAX_TILES = 512;       // query tiles of a sequence: 32768 tokens
@@ -836,7 +911,6 @@ tele_band_dx_kernel(const __grid_constant__ CUtensorMap tmG, const BP p) {
     float* col = cells + tid;
 #pragma unroll
     for (int c = 2; c < SEG + 2; ++c) col[c * BUILDERS] = 0.f;
-    const float last_entry = (float)(p.K - 1);
     Query rec;
     const bool small = p.K == 16 && p.kvec;                // a quarter of a table row for each of a query's threads, loaded a step ahead
     float4 ahead;
@@ -865,19 +939,10 @@ tele_band_dx_kernel(const __grid_constant__ CUtensorMap tmG, const BP p) {
         stage_table(tab, krow, ok, slot_q, STEP, seg, 4, p.K, p.kvec);
       }
       if (seg == 3) tab[p.K * STEP + slot_q] = 0.f;        // met with weight zero: the last value is entry K - 1, and nothing of the next
-      const Taps t{rec.a.x, rec.a.y, rec.a.z, rec.a.w, rec.b.x, rec.b.y, l, ((bits >> 8) & 0xfff) - 512, (bits >> 20) - 512, rec.kmin, rec.kmax};
+      const Taps t = plan_taps(rec.a, rec.b, rec.kmin, rec.kmax, l);
       if (i + 1 < n) fetch(i + 1);
       builders_sync<BUILDERS>();
-      const float* trow = tab + slot_q;
-      const float step_entry = t.f * p.inv_rec * last_entry, step_base = t.f * p.invL;
-      const bool any = __any_sync(0xffffffffu, add_taps(col, t, kseg, p.L, [&](int s, float (&w)[2]) {
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const float as = (float)abs(s + j), idx = fminf(as * step_entry, last_entry), m = floor_magic(idx);
-          const float* e = trow + (__float_as_int(m) - MAGIC_BITS) * STEP;
-          w[j] = fmaf(idx - (m - MAGIC), e[STEP] - e[0], e[0]) * exp2f(-expo * log2f(fmaf(as, step_base, 1.f)));
-        }
-      }));
+      const bool any = __any_sync(0xffffffffu, add_taps(col, t, kseg, p.L, tap_weights(p, tab + slot_q, expo, t.f)));
       if (i >= 1) cta_wait(a_free, (i & 1) ^ 1, abort_flag, p.status, ERR_WAIT_SMEM_EMPTY);
       uint8_t* dst = sA + (seg >> 1) * (STEP * 128) + q * 128;
 #pragma unroll
@@ -909,17 +974,27 @@ tele_band_dx_kernel(const __grid_constant__ CUtensorMap tmG, const BP p) {
     const uint32_t lane_off = uint32_t((warp & 3) * 32) << 16;
     const int cols = p.D >= 32 ? p.D / 2 : p.D, first = part * cols;
     const long long at = (((long long)b * p.L + key) * p.H + h) * p.D;
-    for (int c0 = first; c0 < first + cols && c0 < p.D; c0 += 16) {
+    for (int c0 = first; c0 < first + cols; c0 += 16) {
       uint32_t v[16];
       tmem_ld_32x32b_x16(fr.tmem + lane_off + c0, v);
       tmem_ld_wait();
-      if (key < p.L && !*abort_flag) {
-        float o[16];
+      const bool writes = key < p.L && c0 < p.D && !*abort_flag;
+      float o[16];
+      uint32_t bad = 0;
 #pragma unroll
-        for (int k = 0; k < 16; ++k) {
-          o[k] = n > 0 ? __uint_as_float(v[k]) : 0.f;
-          if (!(fabsf(o[k]) <= FLT_MAX)) o[k] = gathered_dx(p, b, h, key, list, n, c0 + k);
-        }
+      for (int k = 0; k < 16; ++k) {
+        o[k] = n > 0 ? __uint_as_float(v[k]) : 0.f;
+        bad |= is_finite(o[k]) ? 0u : 1u << k;
+      }
+      if (!writes) bad = 0;
+      if (builders_any<BUILDERS>(bad != 0)) {
+        float g[16];
+        gathered_dx(p, b, h, k0, list, n, plan, cells, tabs, reinterpret_cast<uint4*>(sA), c0 - first, cols, bad, g);
+#pragma unroll
+        for (int k = 0; k < 16; ++k)
+          if (bad >> k & 1) o[k] = g[k];
+      }
+      if (writes) {
         if (sizeof(TO) == 2) {
           uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(p.dx) + at + c0);
 #pragma unroll
