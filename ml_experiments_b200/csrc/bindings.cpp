@@ -866,6 +866,12 @@ void chk_rows_f32(const Tensor& t, int64_t n, const char* name) {
   TORCH_CHECK(t.is_cuda() && t.scalar_type() == at::kFloat && t.is_contiguous() && t.numel() == n, name, ": contiguous fp32 CUDA tensor of ", n, " elements");
 }
 
+// Whether a call with these operands (dense; y: the output or its gradient) goes to the band products
+bool tele_band_takes(const Tensor& x, const Tensor& y, int64_t H, int64_t K, int64_t half, double max_rec, bool backward) {
+  const int L = (int)x.size(1), C = (int)x.size(2);
+  return b200::tele_band_takes(x.data_ptr(), y.data_ptr(), (int)x.size(0), L, (int)H, C / (int)H, (int)K, (int)half, (float)max_rec, backward);
+}
+
 void tele_fused_fwd(const Tensor& x, const Tensor& freq, const Tensor& phase, const Tensor& kern, const Tensor& expo, Tensor out,
                     int64_t H, int64_t half, double max_rec, const Tensor& status) {
   const c10::cuda::CUDAGuard guard(x.device());
@@ -1241,6 +1247,7 @@ TORCH_LIBRARY(b200, m) {
   m.def("lincomb3_bwd(Tensor x, Tensor y, Tensor? z, Tensor c, Tensor dout, Tensor(a!) dx, Tensor(b!) dy, Tensor(c!)? dz, Tensor(d!) dc) -> ()");
   m.def("rms_act_fwd(Tensor x, Tensor w, Tensor(a!) y, Tensor(b!) rstd, float eps, int act) -> ()");
   m.def("rms_act_bwd(Tensor x, Tensor w, Tensor rstd, Tensor dy, Tensor? dres, Tensor? dlead, Tensor(a!) dx, Tensor(b!) dw, int act) -> ()");
+  m.def("tele_band_takes(Tensor x, Tensor y, int H, int K, int half, float max_rec, bool backward) -> bool");
   m.def("tele_fused_fwd(Tensor x, Tensor freq, Tensor phase, Tensor kern, Tensor expo, Tensor(a!) out, int H, int half, float max_rec, Tensor(b!) status) -> ()");
   m.def("tele_fused_bwd(Tensor x, Tensor freq, Tensor phase, Tensor kern, Tensor expo, Tensor dout, int H, int half, float max_rec, bool dx_f32, Tensor(a!) status) -> (Tensor, Tensor, Tensor, Tensor, Tensor)");
   m.def("alc_fused_fwd(Tensor x, Tensor half_w, Tensor center, Tensor kern, Tensor(a!) out, int H, int half) -> ()");
@@ -1317,6 +1324,7 @@ TORCH_LIBRARY_IMPL(b200, CUDA, m) {
   m.impl("lincomb3_bwd", &lincomb3_bwd);
   m.impl("rms_act_fwd", &rms_act_fwd);
   m.impl("rms_act_bwd", &rms_act_bwd);
+  m.impl("tele_band_takes", &tele_band_takes);
   m.impl("tele_fused_fwd", &tele_fused_fwd);
   m.impl("tele_fused_bwd", &tele_fused_bwd);
   m.impl("alc_fused_fwd", &alc_fused_fwd);

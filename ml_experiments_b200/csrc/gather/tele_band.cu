@@ -21,6 +21,7 @@
 
 #include <cfloat>
 #include <climits>
+#include <cmath>
 #include <stdexcept>
 #include <string>
 
@@ -1063,17 +1064,22 @@ bool tele_band_takes(const void* x, const void* y, int B, int L, int H, int D, i
   if (need > 232448 - 7168) return false;                  // beside the static part; half <= 119 or 120, 16900 tokens at the operator's own tap count
   if (((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) != 0) return false;
   if ((long long)B * H * ((L + STEP - 1) / STEP) >= (1ll << 31)) return false;
-  // The band grows with the strides, of which max_rec / half is the bound that the caller knows; the gather does not. 2 x 16384 x 4
-  // heads, forward and backward: 16 wide at 22 1.32, 1.43 ms; 32 wide at 32 1.67, 2.00; 64 wide at 48 2.19, 3.57; 128 wide 2.62, 6.7.
+  // The band grows with the strides, of which max_rec / half is the bound that the caller knows; the gather does not.
   if (!(max_rec > 0.f) || max_rec > (D == 16 ? 22.f : D == 32 ? 32.f : 48.f) * half) return false;
-  // Little work: a block of 128 queries takes 10 us forward and 27 backward however few there are, and a gather of narrow rows is cheap.
-  const int taps = 2 * half + 1;
-  const double gathered = (double)B * L * H * taps;
-  // Forward: 256 x 2 heads of 64 10.7, 9.0 us; 600 x 4 of 128 17.5, 13.3 (0.09 M taps); 8 x 256 x 4 of 128 12.8, 16.9 (0.19 M); narrower
-  // heads win from 256 tokens on.
-  if (!backward) return D <= 32 || gathered >= 1.5e5;
-  // Backward: 1500 x 4 heads of 64 (61 taps) 54, 51 us; 8 x 600 x 4 of 16 (37 taps) 59, 44; 4000 x 4 of 16 (107 taps) 79, 87.
-  return taps >= 100 || (D >= 32 && gathered * D >= 5e7);
+  // What is left by estimates of both times in us, fitted to 1896 calls of 128 to 16384 tokens, 1 to 8 heads, tables of 4 to 64 values, strides up
+  // to 16 (10 to 14 % off, root mean square). A gather takes the taps of a row one after the other, or the time of all rows' taps where there are
+  // many; a band as many rounds as there are blocks of 128 rows for 148 multiprocessors, each of its steps of 64 keys, taps and table values
+  // (a table of no multiple of four is read value by value). Of these and 1400 others, 13 that go to the band are more than 3 % slower there,
+  // by 16 % at most; all take 0.73 (forward) and 0.79 of the gather's time on average. Gather and band, backward: 8 x 16384 x 4 heads of 64, table of 64
+  // 10130, 4300 us; 1200 tokens, a head of 128, 33 62, 105; 6000 x 4 of 16, 33 142, 208.
+  const int w = D == 16 ? 0 : D == 32 ? 1 : D == 64 ? 2 : 3;
+  static constexpr double TAP[2][4] = {{0.48, 0.36, 0.30, 0.31}, {0.63, 0.53, 0.47, 0.36}}, ROW_TAP[2][4] = {{13e-6, 19e-6, 34e-6, 63e-6}, {35e-6, 51e-6, 92e-6, 173e-6}};
+  static constexpr double KEYS[2][4] = {{0.60, 0.60, 0.62, 0.90}, {1.75, 1.80, 1.95, 2.15}};
+  const double taps = 2 * half + 1, rows = (double)B * L * H, steps = fmin(128 + 2.0 * max_rec, L) / STEP;
+  const double rounds = fmax(1.0, (double)B * H * ((L + ROWS - 1) / ROWS) / 148 * (backward ? 1.05 : half > 118 ? 1.25 : 1.0));   // (above: one block fits)
+  const double gather = (backward ? 19.0 : 6.5) + fmax(TAP[backward][w] * taps, ROW_TAP[backward][w] * rows * taps);
+  const double band = backward ? 25.5 + rounds * (KEYS[1][w] * steps + 0.145 * taps + (K % 4 ? 0.387 : 0.215) * K) : 11.5 + rounds * (KEYS[0][w] * steps + 0.06 * taps + 0.012 * K);
+  return 1.1 * band < gather;
 }
 
 void tele_band_fwd(const void* x, const float* freq, const float* phase, const float* kern, const float* expo, void* out, int B, int L, int H,

@@ -44,16 +44,39 @@ def _band_inputs(B, L, H, D, K, seed, freq):
     return [t.to("cuda") for t in (x, f, phase, kern, expo)], torch.randn(B, L, H * D, generator=g).bfloat16().float().to("cuda")
 
 
+def _by_band(B, L, H, D, K, half, max_rec=None):
+    """Whether the band products take a call, forward and backward."""
+    from ml_experiments_b200.ops.runtime import ops
+
+    x = torch.empty(B, L, H * D, device="cuda", dtype=torch.bfloat16)
+    return tuple(ops().tele_band_takes(x, x, H, K, half, half * 16.0 if max_rec is None else max_rec, back) for back in (False, True))
+
+
+@pytest.mark.parametrize("B,L,H,D,K,half,fwd,bwd", [
+    (8, 16384, 4, 64, 16, 117, True, True), (8, 16384, 4, 64, 64, 117, True, True),                     # 3570, 1120 us and 10350, 3400; 10130, 4300
+    (1, 1200, 1, 128, 33, 52, True, False), (1, 2000, 1, 64, 64, 70, True, False),                      # backward 62, 105 us and 85, 130
+    (1, 6000, 4, 16, 33, 66, True, False), (8, 16384, 4, 16, 64, 119, False, False),                    # 142, 208; forward 1300, 1617
+    (8, 700, 8, 16, 64, 19, False, False), (2, 3001, 8, 32, 16, 45, True, True)])                        # forward 33, 43; both 96, 74 and 239, 200
+def test_telephone_goes_the_faster_way(B, L, H, D, K, half, fwd, bwd):
+    """Calls for which both were timed (gather, band products), large tables and few blocks among them."""
+    assert _by_band(B, L, H, D, K, half) == (fwd, bwd)
+
+
 @pytest.mark.parametrize("B,L,H,D,K,half,freq", [
     (12, 128, 1, 64, 16, 50, "wide"), (2, 129, 2, 32, 16, 57, "wide"), (1, 191, 4, 16, 64, 59, "signed"), (8, 193, 1, 128, 33, 61, "narrow"),
     (2, 1000, 3, 64, 16, 54, "zero"), (1, 2051, 2, 128, 64, 51, "signed"), (1, 3001, 2, 32, 16, 55, "wide"), (1, 2500, 1, 64, 2, 117, "narrow"),
-    (1, 2500, 1, 128, 6, 118, "wide"), (2, 1201, 4, 64, 16, 37, "wide"), (1, 300, 2, 64, 16, 4, "wide")])
+    (1, 2500, 1, 128, 6, 118, "wide"), (2, 1201, 4, 64, 16, 37, "wide"), (1, 300, 2, 64, 16, 4, "wide"),
+    (6, 2051, 2, 128, 64, 51, "signed"), (5, 3001, 2, 32, 16, 55, "wide"), (6, 2500, 1, 64, 2, 117, "narrow"), (4, 2500, 1, 128, 6, 118, "wide"),
+    (8, 601, 4, 64, 64, 20, "wide"), (8, 577, 2, 128, 47, 60, "zero"), (16, 193, 2, 128, 33, 61, "narrow"), (4, 1000, 3, 64, 16, 54, "zero")])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_telephone_band(B, L, H, D, K, half, freq, dtype):
     """Edges of the tiles of 128 rows and 64 keys, tables that are no multiple of four, strides below one (several taps on a row), negative
-    and zero ones, results in both precisions; the last one is too little work for the products and is gathered."""
+    and zero ones, results in both precisions. Those in `gathered` are too little work for the products, forward or backward."""
     from ml_experiments_b200.ops import fused_taps as T
 
+    gathered = {(1, 2051, 2, 128, 64, 51): (1, 1), (1, 3001, 2, 32, 16, 55): (0, 1), (1, 2500, 1, 64, 2, 117): (0, 1), (1, 2500, 1, 128, 6, 118): (0, 1),
+                (8, 193, 1, 128, 33, 61): (0, 1), (2, 1000, 3, 64, 16, 54): (0, 1), (1, 300, 2, 64, 16, 4): (1, 1)}
+    assert _by_band(B, L, H, D, K, half) == tuple(not g for g in gathered.get((B, L, H, D, K, half), (0, 0)))
     ins, dout = _band_inputs(B, L, H, D, K, L + D, freq)
     leaves = [t.clone().to(dtype if i == 0 else t.dtype).requires_grad_(True) for i, t in enumerate(ins)]
     ref = [t.clone().requires_grad_(True) for t in ins]
@@ -67,7 +90,7 @@ def test_telephone_band(B, L, H, D, K, half, freq, dtype):
         assert _rel(a.grad, b.grad) < tol, (name, _rel(a.grad, b.grad), tol)
 
 
-@pytest.mark.parametrize("D,H", [(16, 4), (64, 2), (128, 2)])
+@pytest.mark.parametrize("D,H", [(16, 4), (64, 4), (128, 4)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_telephone_band_weights_have_24_bits(D, H, dtype):
     """Two rows of opposite sign and nothing else: a result is the difference of the weights of two neighbouring taps, 6.8e-5 of them. It is
@@ -75,12 +98,14 @@ def test_telephone_band_weights_have_24_bits(D, H, dtype):
     from ml_experiments_b200.ops import fused_taps as T
 
     L, K, half, j = 1000, 16, 54, 500
-    pair = torch.zeros(1, L, H * D, device="cuda", dtype=dtype)
+    B = 4
+    assert _by_band(B, L, H, D, K, half) == (True, True)
+    pair = torch.zeros(B, L, H * D, device="cuda", dtype=dtype)
     pair[:, j], pair[:, j + 1] = 1, -1
     x = pair.clone().requires_grad_()
-    one, zero = torch.ones(1, L, H, device="cuda"), torch.zeros(1, L, H, device="cuda")
-    kern = (1 + torch.arange(K, device="cuda") / 256).expand(1, L, H, K).contiguous()
-    y = T.telephone_gather(x, one, zero, kern, torch.zeros(1, L, 1, device="cuda"), H, half, half * 16.0)
+    one, zero = torch.ones(B, L, H, device="cuda"), torch.zeros(B, L, H, device="cuda")
+    kern = (1 + torch.arange(K, device="cuda") / 256).expand(B, L, H, K).contiguous()
+    y = T.telephone_gather(x, one, zero, kern, torch.zeros(B, L, 1, device="cuda"), H, half, half * 16.0)
     y.backward(pair)
     tap = (torch.arange(L, device="cuda") - j).abs().double()
     step = (K - 1) / (half * 16.0) / 256
@@ -90,12 +115,14 @@ def test_telephone_band_weights_have_24_bits(D, H, dtype):
         assert ((got[0, both].double() - want[both, None]).abs() / step).max().item() < 1e-2
 
 
-def test_telephone_band_keeps_what_is_not_finite_where_it_is_sampled():
+@pytest.mark.parametrize("B", [1, 4])
+def test_telephone_band_keeps_what_is_not_finite_where_it_is_sampled(B):
     """A row of x (of the gradient) that is not finite reaches the queries that sample it (the rows that it samples) and no others,
     although products with weights of zero are formed."""
     from ml_experiments_b200.ops import fused_taps as T
 
-    B, L, H, D, half = 1, 700, 2, 64, 54
+    L, H, D, half = 700, 2, 64, 54
+    assert _by_band(B, L, H, D, 16, half) == (True, B == 4)
     ins, dout = _band_inputs(B, L, H, D, 16, 5, "wide")
     ins[0][0, 350, 3] = float("nan")
     ins[0][0, 200, 70] = float("inf")
@@ -115,13 +142,14 @@ def test_telephone_band_keeps_what_is_not_finite_where_it_is_sampled():
     assert _rel(dx[~bad], dxr[~bad]) < 2e-4
 
 
-@pytest.mark.parametrize("B,L,H,D,K", [(1, 4001, 4, 64, 16), (1, 3000, 4, 16, 33), (2, 3000, 2, 128, 64)])
+@pytest.mark.parametrize("B,L,H,D,K", [(1, 4001, 4, 64, 16), (2, 1000, 4, 16, 16), (2, 3000, 2, 128, 64)])
 def test_telephone_band_takes_about_as_long_where_nothing_is_finite(B, L, H, D, K):
     """A step that has diverged: results are formed tap by tap there, until they are no numbers (an element at a time and to the end, it
     took 30 times as long and more)."""
     from ml_experiments_b200.ops import fused_taps as T
 
     half = 54
+    assert _by_band(B, L, H, D, K, half) == (True, True)
     ins, dout = _band_inputs(B, L, H, D, K, 7, "wide")
     ins[0] = ins[0].bfloat16()
 
@@ -155,7 +183,8 @@ def test_telephone_band_strides_that_leave_the_sequence(D, stride):
     gradients are zero. A very large one has tap 0 alone, as 1e6 has."""
     from ml_experiments_b200.ops import fused_taps as T
 
-    B, L, H, half, at = 1, 700, 2, 54, (0, slice(100, 700, 150), 0)
+    B, L, H, half, at = 4, 700, 4, 54, (0, slice(100, 700, 150), 0)
+    assert _by_band(B, L, H, D, 16, half) == (True, True)
     ins, dout = _band_inputs(B, L, H, D, 16, 6, "wide")
     ins[4][0, ::100] *= -1                       # weights that grow with the distance
     grads, ys = [], []
