@@ -1064,7 +1064,7 @@ void rms_act_bwd(const Tensor& x, const Tensor& w, const Tensor& rstd, const Ten
   TORCH_CHECK(norm_io_bf16(dx, "dx") == xb && dx.numel() == x.numel() && dy.numel() == x.numel(), "dx: x's dtype and shape; dy: x's shape");
   const int C = (int)x.size(-1);
   const int64_t R = x.numel() / C;
-  chk_norm_weight(w, C); chk_rows_f32(rstd, R, "rstd"); chk_rows_f32(dw, C, "dw");
+  chk_rows_f32(w, C, "weight"); chk_rows_f32(rstd, R, "rstd"); chk_rows_f32(dw, C, "dw");
   const void* res = nullptr;
   if (dres.has_value()) {
     TORCH_CHECK(dres->is_cuda() && dres->is_contiguous() && dres->scalar_type() == x.scalar_type() && dres->numel() == x.numel(),
@@ -1079,7 +1079,7 @@ void rms_act_bwd(const Tensor& x, const Tensor& w, const Tensor& rstd, const Ten
     lead_p = dlead->data_ptr();
     lead = (int)dlead->size(-1);
   }
-  b200::rms_act_bwd(x.data_ptr(), xb, w.data_ptr(), w.scalar_type() == at::kBFloat16, rstd.data_ptr<float>(), dy.data_ptr(), gb, res, lead_p, lead, dx.data_ptr(),
+  b200::rms_act_bwd(x.data_ptr(), xb, w.data_ptr<float>(), rstd.data_ptr<float>(), dy.data_ptr(), gb, res, lead_p, lead, dx.data_ptr(),
                     dw.data_ptr<float>(), R, C, (int)act, cur_stream());
 }
 

@@ -122,7 +122,7 @@ rms_act_fwd_vec_kernel(const bf16* __restrict__ x, const void* __restrict__ w, b
 
 template <typename TI, typename TO, int ACT>
 __global__ void __launch_bounds__(256)
-rms_act_bwd_kernel(const TI* __restrict__ x, const void* __restrict__ w, bool wb, const float* __restrict__ rstd,
+rms_act_bwd_kernel(const TI* __restrict__ x, const float* __restrict__ w, const float* __restrict__ rstd,
                    const TO* __restrict__ dy, const TI* __restrict__ dres, const TO* __restrict__ dlead, int lead,
                    TI* __restrict__ dx, float* __restrict__ dw, long long R, int C) {
   extern __shared__ float s_dw[];  // [C]
@@ -142,21 +142,21 @@ rms_act_bwd_kernel(const TI* __restrict__ x, const void* __restrict__ w, bool wb
     for (int i = 0; i < 8; ++i) {  // the first 256 columns accumulate dw in registers
       const int c = lane + 32 * i;
       if (c < C) {
-        const float xh = ldf(x, base + c) * rs, wc = ldw(w, wb, c);
+        const float xh = ldf(x, base + c) * rs, wc = w[c];
         const float g = gin(c) * act_grad<ACT>(wc * xh);
         dot += g * wc * xh;
         acc[i] += g * xh;
       }
     }
     for (int c = lane + 256; c < C; c += 32) {
-      const float xh = ldf(x, base + c) * rs, wc = ldw(w, wb, c);
+      const float xh = ldf(x, base + c) * rs, wc = w[c];
       const float g = gin(c) * act_grad<ACT>(wc * xh);
       dot += g * wc * xh;
       atomicAdd(&s_dw[c], g * xh);
     }
     dot = warp_sum(dot) * invC;
     for (int c = lane; c < C; c += 32) {
-      const float xh = ldf(x, base + c) * rs, wc = ldw(w, wb, c);
+      const float xh = ldf(x, base + c) * rs, wc = w[c];
       const float g = gin(c) * act_grad<ACT>(wc * xh);
       stf(dx, base + c, rs * (g * wc - xh * dot) + (dres ? ldf(dres, base + c) : 0.f));
     }
@@ -204,7 +204,7 @@ __device__ __forceinline__ uint4 ldg128_again(const void* p) {
 // read twice (the second time from L1): holding a row between the passes costs the registers of the second resident block.
 template <int VPL, int ACT>
 __global__ void __launch_bounds__(256, 2)
-rms_act_bwd_vec_kernel(const bf16* __restrict__ x, const void* __restrict__ w, bool wb, const float* __restrict__ rstd,
+rms_act_bwd_vec_kernel(const bf16* __restrict__ x, const float* __restrict__ w, const float* __restrict__ rstd,
                        const bf16* __restrict__ dy, const bf16* __restrict__ dres, const bf16* __restrict__ dlead, int lead,
                        bf16* __restrict__ dx, float* __restrict__ dw, long long R) {
   constexpr int C = VPL * 256;
@@ -212,7 +212,7 @@ rms_act_bwd_vec_kernel(const bf16* __restrict__ x, const void* __restrict__ w, b
   __shared__ __align__(16) float s_w[C];
   for (int c = threadIdx.x; c < C; c += 256) {
     s_dw[c] = 0.f;
-    s_w[c] = ldw(w, wb, c);
+    s_w[c] = w[c];
   }
   __syncthreads();
   const int lane = threadIdx.x & 31;
@@ -343,7 +343,7 @@ void rms_act_fwd(const void* x, bool x_bf16, const void* w, bool w_bf16, void* y
   chk("rms_act_fwd");
 }
 
-void rms_act_bwd(const void* x, bool x_bf16, const void* w, bool w_bf16, const float* rstd, const void* dy, bool dy_bf16,
+void rms_act_bwd(const void* x, bool x_bf16, const float* w, const float* rstd, const void* dy, bool dy_bf16,
                  const void* dres, const void* dlead, int lead, void* dx, float* dw, long long R, int C, int act,
                  cudaStream_t s) {
   if (dlead == nullptr) lead = 0;
@@ -351,11 +351,11 @@ void rms_act_bwd(const void* x, bool x_bf16, const void* w, bool w_bf16, const f
   if (C < 1 || C > 4096) throw std::runtime_error("rms_act: row length must be in [1, 4096]");
   if (R == 0) return;
   const bool aligned = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(dx) |
-                         reinterpret_cast<uintptr_t>(dres)) & 15) == 0;
+                         reinterpret_cast<uintptr_t>(dres) | reinterpret_cast<uintptr_t>(w)) & 15) == 0;
   if (x_bf16 && dy_bf16 && aligned && C % 256 == 0 && C <= 1024) {
     const int grid = (int)std::min<long long>((R + 7) / 8, 148LL * 4);
 #define RMS_VEC(VPL_)                                                                                                  \
-  DISPATCH_ACT(act, rms_act_bwd_vec_kernel<VPL_, ACT_><<<grid, 256, 0, s>>>((const bf16*)x, w, w_bf16, rstd, (const bf16*)dy,  \
+  DISPATCH_ACT(act, rms_act_bwd_vec_kernel<VPL_, ACT_><<<grid, 256, 0, s>>>((const bf16*)x, w, rstd, (const bf16*)dy,  \
                                                                              (const bf16*)dres, (const bf16*)dlead, lead,    \
                                                                              (bf16*)dx, dw, R))
     switch (C / 256) {
@@ -369,7 +369,7 @@ void rms_act_bwd(const void* x, bool x_bf16, const void* w, bool w_bf16, const f
     return;
   }
   DISPATCH_ACT(act, DISPATCH_IO(x_bf16, dy_bf16, {
-    rms_act_bwd_kernel<TI_, TO_, ACT_><<<grid_for(R), 256, (size_t)C * sizeof(float), s>>>((const TI_*)x, w, w_bf16, rstd, (const TO_*)dy, (const TI_*)dres, (const TO_*)dlead, lead, (TI_*)dx, dw, R, C);
+    rms_act_bwd_kernel<TI_, TO_, ACT_><<<grid_for(R), 256, (size_t)C * sizeof(float), s>>>((const TI_*)x, w, rstd, (const TO_*)dy, (const TI_*)dres, (const TO_*)dlead, lead, (TI_*)dx, dw, R, C);
   }));
   chk("rms_act_bwd");
 }

@@ -21,21 +21,28 @@ def rms_norm_act_ref(x, weight, eps: float = 1e-6, act: str = "none", out_dtype=
     return y.to(out_dtype or x.dtype)
 
 
-def _weight(w):
-    """The weight as the kernels read it: dense, fp32 or bf16."""
+def _weight(w, keep):
+    """The weight as the kernels read it: dense and, where it is kept for a backward, its fp32 values (the parameter itself may change
+    before that comes); a forward alone reads bf16 weights as they are."""
     w = w.detach()
-    return (w if w.dtype in (torch.float32, torch.bfloat16) else w.float()).contiguous()
+    return (w if w.dtype == torch.bfloat16 and not keep else w.float()).contiguous()
+
+
+def _keeps(x, weight):
+    # (asked outside of the functions: inside, gradients are always off)
+    return torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad)
 
 
 class _RmsAct(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, weight, eps, act, out_dtype):
+    def forward(ctx, x, weight, eps, act, out_dtype, keep):
         xc = x.contiguous()
-        w = _weight(weight)
+        w = _weight(weight, keep)
         y = torch.empty(xc.shape, dtype=out_dtype, device=x.device)
         rstd = torch.empty(xc.numel() // xc.shape[-1], dtype=torch.float32, device=x.device)
         ops().rms_act_fwd(xc, w, y, rstd, eps, act)
-        ctx.save_for_backward(xc, w, rstd)
+        if keep:
+            ctx.save_for_backward(xc, w, rstd)
         ctx.act, ctx.wdtype = act, weight.dtype
         return y
 
@@ -45,9 +52,9 @@ class _RmsAct(torch.autograd.Function):
         if dy.dtype not in (torch.bfloat16, torch.float32):
             dy = dy.float()
         dx = torch.empty_like(xc)
-        dw = torch.zeros(w.shape, dtype=torch.float32, device=w.device)
+        dw = torch.zeros_like(w)
         ops().rms_act_bwd(xc, w, rstd, dy.contiguous(), None, None, dx, dw, ctx.act)
-        return dx, dw.to(ctx.wdtype), None, None, None
+        return dx, dw.to(ctx.wdtype), None, None, None, None
 
 
 class _RmsActSkip(torch.autograd.Function):
@@ -58,13 +65,14 @@ class _RmsActSkip(torch.autograd.Function):
     instead of a zero-filled full-size tensor and another add."""
 
     @staticmethod
-    def forward(ctx, x, weight, eps, act, lead):
+    def forward(ctx, x, weight, eps, act, lead, keep):
         xc = x.contiguous()
-        w = _weight(weight)
+        w = _weight(weight, keep)
         y = torch.empty_like(xc)
         rstd = torch.empty(xc.numel() // xc.shape[-1], dtype=torch.float32, device=x.device)
         ops().rms_act_fwd(xc, w, y, rstd, eps, act)
-        ctx.save_for_backward(xc, w, rstd)
+        if keep:
+            ctx.save_for_backward(xc, w, rstd)
         ctx.act, ctx.wdtype, ctx.lead = act, weight.dtype, lead
         if lead:
             return y, x.view_as(x), y[..., :lead].contiguous()
@@ -76,10 +84,10 @@ class _RmsActSkip(torch.autograd.Function):
         if dy.dtype not in (torch.bfloat16, torch.float32):
             dy = dy.float()
         dx = torch.empty_like(xc)
-        dw = torch.zeros(w.shape, dtype=torch.float32, device=w.device)
+        dw = torch.zeros_like(w)
         lead = dlead.to(dy.dtype).contiguous() if (ctx.lead and dlead is not None) else None
         ops().rms_act_bwd(xc, w, rstd, dy.contiguous(), dskip.to(xc.dtype).contiguous(), lead, dx, dw, ctx.act)
-        return dx, dw.to(ctx.wdtype), None, None, None
+        return dx, dw.to(ctx.wdtype), None, None, None, None
 
 
 def rms_norm_act(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6, act: str = "none", out_dtype=None) -> torch.Tensor:
@@ -88,7 +96,7 @@ def rms_norm_act(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6, act: 
           and 1 <= x.shape[-1] <= 4096 and weight.numel() == x.shape[-1])
     if not ok:
         return rms_norm_act_ref(x, weight, eps, act, out_dtype)
-    return _RmsAct.apply(x, weight, float(eps), _ACTS[act], out_dtype)
+    return _RmsAct.apply(x, weight, float(eps), _ACTS[act], out_dtype, _keeps(x, weight))
 
 
 def rms_norm_act_skip(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6, act: str = "none", lead_cols: int = 0):
@@ -99,4 +107,4 @@ def rms_norm_act_skip(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6, 
     if not ok:
         y = rms_norm_act_ref(x, weight, eps, act)
         return (y, x, y[..., :lead_cols]) if lead_cols else (y, x)
-    return _RmsActSkip.apply(x, weight, float(eps), _ACTS[act], int(lead_cols))
+    return _RmsActSkip.apply(x, weight, float(eps), _ACTS[act], int(lead_cols), _keeps(x, weight))

@@ -267,6 +267,28 @@ def test_rms_norm_act_with_bf16_weights_is_the_same_as_with_their_fp32_values(C,
     assert torch.equal(xa.grad, xb.grad) and wa.grad.dtype == torch.bfloat16 and _rel(wa.grad, wb.grad) < 4e-3
 
 
+def test_rms_norm_act_bf16_weights_may_change_before_the_backward():
+    """An optimizer may step between a forward and its backward: the gradients are those of the weights that the forward had."""
+    from ml_experiments_b200.ops.norm_act import rms_norm_act, rms_norm_act_skip
+
+    g = torch.Generator().manual_seed(3)
+    for C in (512, 300):
+        x = torch.randn(50, C, generator=g).bfloat16().cuda()
+        w = (torch.rand(C, generator=g) + 0.5).bfloat16().cuda()
+        gy = torch.randn(50, C, generator=g).bfloat16().cuda()
+        for norm in (lambda a, b: rms_norm_act(a, b, 1e-6, "silu"), lambda a, b: rms_norm_act_skip(a, b, 1e-6, "silu")[0]):
+            grads = []
+            for change in (False, True):
+                xa, wa = x.clone().requires_grad_(), w.clone().requires_grad_()
+                y = norm(xa, wa)
+                if change:
+                    with torch.no_grad():
+                        wa.mul_(3)
+                y.backward(gy)
+                grads.append((xa.grad, wa.grad))
+            assert torch.equal(grads[0][0], grads[1][0]) and _rel(grads[1][1], grads[0][1]) < 4e-3     # (dw: sums in any order)
+
+
 @pytest.mark.parametrize("C,dtype,lead", [(768, torch.bfloat16, 12), (1024, torch.bfloat16, 0), (512, torch.bfloat16, 9), (300, torch.bfloat16, 12),
                                           (256, torch.float32, 5)])
 def test_rms_norm_act_skip_adds_the_skip_gradient_in_the_backward_kernel(C, dtype, lead):
