@@ -15,10 +15,6 @@ using bf16 = __nv_bfloat16;
 template <typename T> __device__ __forceinline__ float ldf(const T* p, long long i);
 template <> __device__ __forceinline__ float ldf<float>(const float* p, long long i) { return p[i]; }
 template <> __device__ __forceinline__ float ldf<bf16>(const bf16* p, long long i) { return __bfloat162float(p[i]); }
-// weight c, fp32 or bf16
-__device__ __forceinline__ float ldw(const void* w, bool wb, int c) {
-  return wb ? __bfloat162float(reinterpret_cast<const bf16*>(w)[c]) : reinterpret_cast<const float*>(w)[c];
-}
 template <typename T> __device__ __forceinline__ void stf(T* p, long long i, float v);
 template <> __device__ __forceinline__ void stf<float>(float* p, long long i, float v) { p[i] = v; }
 template <> __device__ __forceinline__ void stf<bf16>(bf16* p, long long i, float v) { p[i] = __float2bfloat16(v); }
@@ -53,9 +49,9 @@ __device__ __forceinline__ float act_grad(float u) {
   return 1.f;
 }
 
-template <typename TI, typename TO, int ACT>
+template <typename TI, typename TO, typename TW, int ACT>
 __global__ void __launch_bounds__(256)
-rms_act_fwd_kernel(const TI* __restrict__ x, const void* __restrict__ w, bool wb, TO* __restrict__ y, float* __restrict__ rstd,
+rms_act_fwd_kernel(const TI* __restrict__ x, const TW* __restrict__ w, TO* __restrict__ y, float* __restrict__ rstd,
                    long long R, int C, float eps) {
   const int lane = threadIdx.x & 31;
   const long long warps = (long long)gridDim.x * 8;
@@ -68,16 +64,16 @@ rms_act_fwd_kernel(const TI* __restrict__ x, const void* __restrict__ w, bool wb
     }
     const float rs = rsqrtf(warp_sum(ss) / (float)C + eps);
     if (lane == 0) rstd[row] = rs;
-    for (int c = lane; c < C; c += 32) stf(y, base + c, act_fwd<ACT>(ldw(w, wb, c) * ldf(x, base + c) * rs));
+    for (int c = lane; c < C; c += 32) stf(y, base + c, act_fwd<ACT>(ldf(w, c) * ldf(x, base + c) * rs));
   }
 }
 
 // Forward for bf16 rows of 256 * VPL columns: a lane moves groups of 8 columns with 16-byte accesses and keeps its part of the row, which is
 // read once, and of the weights, which are read once per warp. Bound: memory, one read and one write of the rows.
 // 32768 x 1024: 22 us (31 us with a column per lane and access and two reads).
-template <int VPL, int ACT>
+template <int VPL, typename TW, int ACT>
 __global__ void __launch_bounds__(256)
-rms_act_fwd_vec_kernel(const bf16* __restrict__ x, const void* __restrict__ w, bool wb, bf16* __restrict__ y, float* __restrict__ rstd, long long R,
+rms_act_fwd_vec_kernel(const bf16* __restrict__ x, const TW* __restrict__ w, bf16* __restrict__ y, float* __restrict__ rstd, long long R,
                        float eps) {
   constexpr int C = VPL * 256;
   const int lane = threadIdx.x & 31;
@@ -85,7 +81,7 @@ rms_act_fwd_vec_kernel(const bf16* __restrict__ x, const void* __restrict__ w, b
 #pragma unroll
   for (int j = 0; j < VPL; ++j)
 #pragma unroll
-    for (int e = 0; e < 8; ++e) wv[j][e] = ldw(w, wb, (j * 32 + lane) * 8 + e);
+    for (int e = 0; e < 8; ++e) wv[j][e] = ldf(w, (j * 32 + lane) * 8 + e);
   const long long warps = (long long)gridDim.x * 8;
   for (long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); row < R; row += warps) {
     const uint4* src = reinterpret_cast<const uint4*>(x + row * C) + lane;
@@ -318,15 +314,11 @@ int grid_for(long long R) {
   else if (xb && !yb) { using TI_ = bf16; using TO_ = float; __VA_ARGS__; }        \
   else if (!xb && yb) { using TI_ = float; using TO_ = bf16; __VA_ARGS__; }        \
   else { using TI_ = float; using TO_ = float; __VA_ARGS__; }
-}  // namespace
-
-void rms_act_fwd(const void* x, bool x_bf16, const void* w, bool w_bf16, void* y, bool y_bf16, float* rstd, long long R, int C, float eps,
-                 int act, cudaStream_t s) {
-  if (C < 1 || C > 4096) throw std::runtime_error("rms_act: row length must be in [1, 4096]");
-  if (R == 0) return;
+template <typename TW>
+void fwd_by_weights(const void* x, bool x_bf16, const TW* w, void* y, bool y_bf16, float* rstd, long long R, int C, float eps, int act, cudaStream_t s) {
   const bool even = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
   if (x_bf16 && y_bf16 && even && C % 256 == 0 && C <= 1024) {
-#define RMS_VEC(VPL_) DISPATCH_ACT(act, rms_act_fwd_vec_kernel<VPL_, ACT_><<<grid_for(R), 256, 0, s>>>((const bf16*)x, w, w_bf16, (bf16*)y, rstd, R, eps))
+#define RMS_VEC(VPL_) DISPATCH_ACT(act, rms_act_fwd_vec_kernel<VPL_, TW, ACT_><<<grid_for(R), 256, 0, s>>>((const bf16*)x, w, (bf16*)y, rstd, R, eps))
     switch (C / 256) {
       case 1: RMS_VEC(1); break;
       case 2: RMS_VEC(2); break;
@@ -334,12 +326,20 @@ void rms_act_fwd(const void* x, bool x_bf16, const void* w, bool w_bf16, void* y
       default: RMS_VEC(4); break;
     }
 #undef RMS_VEC
-    chk("rms_act_fwd");
     return;
   }
   DISPATCH_ACT(act, DISPATCH_IO(x_bf16, y_bf16, {
-    rms_act_fwd_kernel<TI_, TO_, ACT_><<<grid_for(R), 256, 0, s>>>((const TI_*)x, w, w_bf16, (TO_*)y, rstd, R, C, eps);
+    rms_act_fwd_kernel<TI_, TO_, TW, ACT_><<<grid_for(R), 256, 0, s>>>((const TI_*)x, w, (TO_*)y, rstd, R, C, eps);
   }));
+}
+}  // namespace
+
+void rms_act_fwd(const void* x, bool x_bf16, const void* w, bool w_bf16, void* y, bool y_bf16, float* rstd, long long R, int C, float eps,
+                 int act, cudaStream_t s) {
+  if (C < 1 || C > 4096) throw std::runtime_error("rms_act: row length must be in [1, 4096]");
+  if (R == 0) return;
+  if (w_bf16) fwd_by_weights(x, x_bf16, (const bf16*)w, y, y_bf16, rstd, R, C, eps, act, s);
+  else fwd_by_weights(x, x_bf16, (const float*)w, y, y_bf16, rstd, R, C, eps, act, s);
   chk("rms_act_fwd");
 }
 
