@@ -151,13 +151,16 @@ class _S6Inner(torch.autograd.Function):
         o.s6_join_bc(parts, ddbc)
         del parts
         dd2, u2 = ddelta.view(-1, c), u.view(-1, c)
+        dx_w = ddt_w = None
         G.gemm(dd2, dt_w16, b_mn=True, out=ddbc[:, :r])
-        ddt_w = G.gemm(dd2, dbc[:, :r], a_mn=True, b_mn=True, split_k=G.auto_split_k(c, r, dd2.shape[0]), out_dtype=torch.float32)
+        if ctx.needs_input_grad[5]:
+            ddt_w = G.gemm(dd2, dbc[:, :r], a_mn=True, b_mn=True, split_k=G.auto_split_k(c, r, dd2.shape[0]), out_dtype=torch.float32).to(ctx.dtypes[1])
         du = G.gemm(ddbc, x_w16, b_mn=True, epilogue=G.EPI_AXPBY, aux=du.view(-1, c), alpha=1.0, beta=1.0)
-        dx_w = G.gemm(ddbc, u2, a_mn=True, b_mn=True, split_k=G.auto_split_k(ddbc.shape[1], c, u2.shape[0]), out_dtype=torch.float32)
+        if ctx.needs_input_grad[4]:
+            dx_w = G.gemm(ddbc, u2, a_mn=True, b_mn=True, split_k=G.auto_split_k(ddbc.shape[1], c, u2.shape[0]), out_dtype=torch.float32).to(ctx.dtypes[0])
         o.causal_conv1d_silu_bwd(xi, taps, bias, du.view(bsz, L, c), dxi, dtaps, dbias)
         dcw, dcb, dal, dd, ddb = o.s6_param_grads(params, grads, packed)
-        return dxi, dz, dcw.view(ctx.shapes), dcb, dx_w.to(ctx.dtypes[0]), ddt_w.to(ctx.dtypes[1]), ddb, dal, dd, None
+        return dxi, dz, dcw.view(ctx.shapes), dcb, dx_w, ddt_w, ddb, dal, dd, None
 
 
 def _s6_views(packed, c):

@@ -259,6 +259,34 @@ def test_s6_inner_is_convolution_projections_and_scan(bsz, L, c, rank, dtype):
         assert torch.equal(s6_inner(*a), y)
 
 
+def _mixer_backward(frozen=(), change=(), dtype=torch.bfloat16):
+    """Gradients of a mixer's input and parameters and the launches of its backward; ``change``: parameters that are tripled before it."""
+    from ml_experiments_b200.models.s6 import S6Config, S6Mixer
+    from ml_experiments_b200.ops.runtime import launch_count
+
+    torch.manual_seed(5)
+    m = S6Mixer(S6Config(d_model=128, n_layers=1)).cuda().to(dtype)
+    x = torch.randn(2, 100, 128, device="cuda").bfloat16().requires_grad_()
+    params = dict(m.named_parameters())
+    for n in frozen:
+        params[n].requires_grad_(False)
+    y = m(x)
+    with torch.no_grad():
+        for n in change:
+            params[n].mul_(3)
+    before = launch_count()
+    (y.float() * torch.randn(y.shape, device="cuda")).sum().backward()
+    return {"x": x.grad, **{n: p.grad for n, p in params.items()}}, launch_count() - before
+
+
+def test_s6_inner_forms_no_gradients_of_frozen_projections():
+    want, full = _mixer_backward()
+    for frozen in (["x_proj.weight"], ["dt_proj.weight"], ["x_proj.weight", "dt_proj.weight"]):
+        got, launches = _mixer_backward(frozen)
+        assert launches == full - len(frozen)
+        assert all(got[n] is None if n in frozen else torch.allclose(got[n].float(), g.float(), rtol=2e-2, atol=1e-3 * g.abs().max().item()) for n, g in want.items())
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("din", [16, 1000, 37])          # the pipelined kernels, their last block half full, the general ones
 def test_softplus_of_delta(dtype, din):
