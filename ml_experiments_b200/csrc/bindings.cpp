@@ -683,16 +683,13 @@ Tensor s6_params(at::TensorList params) {
   b200::s6_params(s6_tensors(params, C), packed.data_ptr<float>(), (int)C, cur_stream());
   return packed;
 }
-std::vector<Tensor> s6_param_grads(at::TensorList params, const Tensor& grads, const Tensor& packed) {
-  TORCH_CHECK(params.size() == 5, "s6: five parameters");
+void s6_param_grads(at::TensorList out, const Tensor& grads, const Tensor& packed) {
+  TORCH_CHECK(out.size() == 5, "s6: five parameters");
   const c10::cuda::CUDAGuard guard(grads.device());
-  const int64_t C = params[3].numel();
+  const int64_t C = out[3].numel();
   for (const Tensor& t : {grads, packed})
     TORCH_CHECK(t.is_cuda() && t.is_contiguous() && t.scalar_type() == at::kFloat && t.numel() == 23 * C, "s6: gradients and packed parameters: fp32 [23 C]");
-  std::vector<Tensor> out;
-  for (const Tensor& p : params) out.push_back(at::empty_like(p));
   b200::s6_param_grads(s6_tensors(out, C), grads.data_ptr<float>(), packed.data_ptr<float>(), (int)C, cur_stream());
-  return out;
 }
 void chk_dbc(const Tensor& t, const char* name) {
   chk_bf16c(t, name);
@@ -1234,7 +1231,7 @@ TORCH_LIBRARY(b200, m) {
   m.def("s6_scan_fwd(Tensor u, Tensor delta, Tensor? delta_bias, bool softplus, Tensor A, Tensor Bm, Tensor Cm, Tensor? Dv, Tensor? z, Tensor(a!)? y_pre, Tensor(b!) out, Tensor(c!)? state) -> ()");
   m.def("s6_scan_bwd(Tensor u, Tensor delta, Tensor? delta_bias, bool softplus, Tensor A, Tensor Bm, Tensor Cm, Tensor? Dv, Tensor? z, Tensor? y_pre, Tensor dout, Tensor state, Tensor(a!) du, Tensor(b!) ddelta, Tensor(c!) dA, Tensor(d!) dB_part, Tensor(e!) dC_part, Tensor(f!)? dD, Tensor(g!)? dz, Tensor(h!)? ddelta_bias) -> ()");
   m.def("s6_params(Tensor[] params) -> Tensor");
-  m.def("s6_param_grads(Tensor[] params, Tensor grads, Tensor packed) -> Tensor[]");
+  m.def("s6_param_grads(Tensor(a!)[] out, Tensor grads, Tensor packed) -> ()");
   m.def("s6_split_bc(Tensor dbc) -> Tensor");
   m.def("s6_join_bc(Tensor parts, Tensor(a!) ddbc) -> ()");
   m.def("causal_conv1d_silu_fwd(Tensor x, Tensor w, Tensor? bias, Tensor(a!) y) -> ()");

@@ -128,15 +128,15 @@ class _S6Inner(torch.autograd.Function):
         out = torch.empty_like(xi)
         o.s6_scan_fwd(u, delta, dtb, True, A, bc[0], bc[1], D32, z, y_pre, out, state)
         if need_grad:
-            ctx.save_for_backward(xi, z, u, dbc, delta, bc, packed, y_pre, state, x_w16, dt_w16, *params)
+            ctx.save_for_backward(xi, z, u, dbc, delta, bc, packed, y_pre, state, x_w16, dt_w16)
         ctx.dtypes = x_w.dtype, dt_w.dtype
-        ctx.shapes = conv_w.shape
+        ctx.small = [(t.shape, t.dtype) for t in (conv_w, conv_b, A_log, D, dt_b)]     # (their values are in `packed`)
         return out
 
     @staticmethod
     def backward(ctx, dout):
         o = ops()
-        xi, z, u, dbc, delta, bc, packed, y_pre, state, x_w16, dt_w16, *params = ctx.saved_tensors
+        xi, z, u, dbc, delta, bc, packed, y_pre, state, x_w16, dt_w16 = ctx.saved_tensors
         bsz, L, c = xi.shape
         r = dt_w16.shape[1]
         dev = xi.device
@@ -159,8 +159,9 @@ class _S6Inner(torch.autograd.Function):
         if ctx.needs_input_grad[4]:
             dx_w = G.gemm(ddbc, u2, a_mn=True, b_mn=True, split_k=G.auto_split_k(ddbc.shape[1], c, u2.shape[0]), out_dtype=torch.float32).to(ctx.dtypes[0])
         o.causal_conv1d_silu_bwd(xi, taps, bias, du.view(bsz, L, c), dxi, dtaps, dbias)
-        dcw, dcb, dal, dd, ddb = o.s6_param_grads(params, grads, packed)
-        return dxi, dz, dcw.view(ctx.shapes), dcb, dx_w, ddt_w, ddb, dal, dd, None
+        dcw, dcb, dal, dd, ddb = small = [torch.empty(s, dtype=d, device=dev) for s, d in ctx.small]
+        o.s6_param_grads(small, grads, packed)
+        return dxi, dz, dcw, dcb, dx_w, ddt_w, ddb, dal, dd, None
 
 
 def _s6_views(packed, c):

@@ -288,6 +288,16 @@ def test_s6_inner_forms_no_gradients_of_frozen_projections():
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_s6_inner_small_parameters_may_change_before_the_backward(dtype):
+    """An optimizer may step between a forward and its backward: the gradients are those of the parameters that the forward had."""
+    change = ["conv1d.weight", "conv1d.bias", "A_log", "D", "dt_proj.bias"]
+    want, _ = _mixer_backward(dtype=dtype)
+    got, _ = _mixer_backward(change=change, dtype=dtype)
+    for n, g in want.items():
+        assert torch.allclose(got[n].float(), g.float(), rtol=2e-2, atol=1e-3 * g.abs().max().item()), n      # (bf16; sums in any order)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("din", [16, 1000, 37])          # the pipelined kernels, their last block half full, the general ones
 def test_softplus_of_delta(dtype, din):
     """dt read off a state checkpoint (no decay, one input) and its derivative off ddelta, against 64 bits, over the range of delta.
