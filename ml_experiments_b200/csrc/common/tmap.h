@@ -92,6 +92,9 @@ inline CUtensorMap encode_tmap_3d(const void* base, TmapDtype dt, uint64_t d0, u
   if ((reinterpret_cast<uintptr_t>(base) & 15) != 0) throw std::runtime_error("TMA base address must be 16-byte aligned");
   if ((strides[0] & 15) != 0 || (strides[1] & 15) != 0)
     throw std::runtime_error("TMA strides must be multiples of 16 bytes (row length * element size)");
+  // The driver's call needs the context to be current, which in a new thread (autograd's, say) it is only after the runtime was asked for it.
+  int dev = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess) (void)cudaSetDevice(dev);
   CUresult r = get_encode_fn()(&m, cdt, 3, const_cast<void*>(base), dims, strides, box, estr,
                                CU_TENSOR_MAP_INTERLEAVE_NONE,
                                swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,

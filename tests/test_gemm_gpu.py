@@ -127,6 +127,27 @@ def test_gemm_fp8_by_pairs():
         assert _rel_err(gemm(a, b, b_mn=b_mn, out_dtype=torch.float32, alpha=0.25), 0.25 * _ref(a, b, False, b_mn)) < 2e-3
 
 
+_BACKWARD_FIRST = """
+import torch
+from ml_experiments_b200.ops.linear import linear
+x, w = (torch.randn(128, 128, device="cuda", dtype=torch.bfloat16, requires_grad=True) for _ in range(2))
+y = linear(x, w)
+y.backward(torch.ones_like(y))
+assert ((x.grad.float() - w.detach().float().sum(0)).abs() < 0.2).all()
+"""
+
+
+def test_a_product_as_the_first_operator_of_a_backward():
+    """The thread of autograd has not touched the device then. (A process of its own: here it has.)"""
+    import os
+    import subprocess
+    import sys
+
+    r = subprocess.run([sys.executable, "-c", _BACKWARD_FIRST], capture_output=True, text=True, timeout=300,
+                       cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert r.returncode == 0, r.stderr[-500:]
+
+
 def test_output_aliasing_an_operand_is_refused():
     """In-place products are a timing-dependent race between CTAs (one stores a tile of the operand another still
     reads); the front end rejects them instead of returning numbers that are right most of the time."""
