@@ -36,6 +36,10 @@ int gemm_dtype(const Tensor& t) {
   }
 }
 
+bool gemm_by_pairs(int64_t M, int64_t N, int64_t K, int64_t batch, bool both_mn, int64_t element_bytes, int64_t splits) {
+  return b200::gemm_by_pairs((int)M, (int)N, (int)K, (int)batch, both_mn, (int)element_bytes, (int)splits);
+}
+
 cudaStream_t cur_stream() { return at::cuda::getCurrentCUDAStream().stream(); }
 
 // c = epilogue(a @ b^T) with per-operand majorness; see csrc/gemm/gemm.h.
@@ -1244,6 +1248,7 @@ TORCH_LIBRARY(b200, m) {
   m.def("lincomb3_bwd(Tensor x, Tensor y, Tensor? z, Tensor c, Tensor dout, Tensor(a!) dx, Tensor(b!) dy, Tensor(c!)? dz, Tensor(d!) dc) -> ()");
   m.def("rms_act_fwd(Tensor x, Tensor w, Tensor(a!) y, Tensor(b!) rstd, float eps, int act) -> ()");
   m.def("rms_act_bwd(Tensor x, Tensor w, Tensor rstd, Tensor dy, Tensor? dres, Tensor? dlead, Tensor(a!) dx, Tensor(b!) dw, int act) -> ()");
+  m.def("gemm_by_pairs(int M, int N, int K, int batch, bool both_mn, int element_bytes, int splits) -> bool", &gemm_by_pairs);
   m.def("tele_band_takes(Tensor x, Tensor y, int H, int K, int half, float max_rec, bool backward) -> bool");
   m.def("tele_fused_fwd(Tensor x, Tensor freq, Tensor phase, Tensor kern, Tensor expo, Tensor(a!) out, int H, int half, float max_rec, Tensor(b!) status) -> ()");
   m.def("tele_fused_bwd(Tensor x, Tensor freq, Tensor phase, Tensor kern, Tensor expo, Tensor dout, int H, int half, float max_rec, bool dx_f32, Tensor(a!) status) -> (Tensor, Tensor, Tensor, Tensor, Tensor)");

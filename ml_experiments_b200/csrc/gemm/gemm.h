@@ -40,5 +40,7 @@ struct GemmArgs {
 
 // Throws std::runtime_error on invalid arguments / launch failure.
 void gemm_sm100(const GemmArgs& args);
+// Whether a product with these sizes, on all multiprocessors, is formed by pairs of CTAs
+bool gemm_by_pairs(int M, int N, int K, int batch, bool both_mn, int element_bytes, int splits);
 
 }  // namespace b200

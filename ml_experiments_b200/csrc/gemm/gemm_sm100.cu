@@ -471,7 +471,7 @@ void dispatch_major(const GemmArgs& a, const KParams& kp, const CUtensorMap& tA,
   if (!a.a_mn && !a.b_mn) launch<BN, STAGES, 0, 0, ESZ, PAIR>(a, kp, tA, tB, tC, tX, grid);
   else if (!a.a_mn && a.b_mn) launch<BN, STAGES, 0, 1, ESZ, PAIR>(a, kp, tA, tB, tC, tX, grid);
   else if (a.a_mn && !a.b_mn) launch<BN, STAGES, 1, 0, ESZ, PAIR>(a, kp, tA, tB, tC, tX, grid);
-  else launch<BN, STAGES, 1, 1, ESZ, PAIR>(a, kp, tA, tB, tC, tX, grid);
+  else if constexpr (!PAIR) launch<BN, STAGES, 1, 1, ESZ, 0>(a, kp, tA, tB, tC, tX, grid);      // (by_pairs: never pairs)
 }
 
 }  // namespace
@@ -479,14 +479,20 @@ void dispatch_major(const GemmArgs& a, const KParams& kp, const CUtensorMap& tA,
 // A pair's set-up and end (clusters, their barriers) take time, and its tiles of 256 rows may leave more of the machine without work in
 // the last round. Weight gradients (both operands MN-major, K long) gain nothing from it: 3072 x 768 x 49152 163, 159 us.
 // Pair, single: 8 of 3072 x 768 x 768 (29 GFLOP) 29.2, 27.5 us; 10007 x 3072 x 768 (47) 39.8, 41.3; 16 of 768 x 768 x
-// 3072 (58) 47.4, 49.5; 20011 x 3072 x 768 72, 77; 49152 x 3072 x 768 173, 186.
-static bool pair_is_faster(const GemmArgs& a, int splits, int sms) {
-  if (a.M <= BM || 2.0 * a.M * a.N * a.K * a.batch < 4e10 || (a.a_mn && a.b_mn)) return false;
+// 3072 (58) 47.4, 49.5; 20011 x 3072 x 768 72, 77; 49152 x 3072 x 768 173, 186. Nor has a pair enough work in a tile whose K ends after a few
+// stages of 128 bytes, where its epilogue, twice as long, is not hidden: bf16, 49152 x 3072 x 256 119, 92, x 512 133, 127; fp8, 49152 x 50304 x 768 2550, 1910.
+// From 11 stages on it is the faster one (bf16: 704 0.97, 640 1.0 of the single's time, means of five sizes and five epilogues).
+static bool by_pairs(int M, int N, int K, int batch, bool both_mn, int esz, int splits, int sms) {
+  if (N <= 128 || sms < 2 || M <= BM || 2.0 * M * N * K * batch < 4e10 || both_mn) return false;
+  if ((K + splits - 1) / splits * esz <= 10 * 128) return false;
   auto rounds = [&](int rows, int at_once) {
-    const long long tiles = (long long)((a.M + rows - 1) / rows) * ((a.N + 255) / 256) * splits * a.batch;
+    const long long tiles = (long long)((M + rows - 1) / rows) * ((N + 255) / 256) * splits * batch;
     return (double)((tiles + at_once - 1) / at_once);
   };
   return 0.9 * rounds(2 * BM, sms / 2) <= rounds(BM, sms);
+}
+bool gemm_by_pairs(int M, int N, int K, int batch, bool both_mn, int element_bytes, int splits) {
+  return by_pairs(M, N, K, batch, both_mn, element_bytes, splits, sm_count());
 }
 
 void gemm_sm100(const GemmArgs& a) {
@@ -505,7 +511,7 @@ void gemm_sm100(const GemmArgs& a) {
 
   const int BN = a.N > 128 ? 256 : 128;
   const int sms = a.max_ctas > 0 ? a.max_ctas : sm_count();
-  const bool pair = BN == 256 && sms >= 2 && pair_is_faster(a, splits, sms);
+  const bool pair = by_pairs(a.M, a.N, a.K, a.batch, a.a_mn && a.b_mn, esz, splits, sms);
   const int TM = pair ? 2 * BM : BM, brows = pair ? BN / 2 : BN;
   const int BK = 128 / esz;
   const int span = 128 / esz;

@@ -94,14 +94,16 @@ def test_gemm_fp8(a_mn, b_mn):
 
 
 @pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, False)])
-@pytest.mark.parametrize("m,n,k,batch", [(8193, 2312, 1096, None), (16384 + 128, 776, 1608, None), (640, 1032, 1032, 33)])
+@pytest.mark.parametrize("m,n,k,batch", [(8193, 2312, 1096, None), (16384 + 128, 776, 1608, None), (640, 1032, 1032, 33), (776, 760, 3080, 16)])
 def test_gemm_by_pairs(a_mn, b_mn, m, n, k, batch):
     """Products large enough for pairs of CTAs on tiles of 256 x 256: a last tile of one row, of one CTA only, of a few columns; a K that
-    is no multiple of a stage; batches; every epilogue."""
+    is no multiple of a stage; batches (33 of them leave too many tiles for the last round: by single CTAs); every epilogue."""
     from ml_experiments_b200.ops import gemm as G
+    from ml_experiments_b200.ops.runtime import ops
 
     m = (m + 7) // 8 * 8 if a_mn else m          # (rows of 16-byte multiples)
     assert 2 * m * n * k * (batch or 1) >= 4e10
+    assert ops().gemm_by_pairs(m, n, k, batch or 1, False, 2, 1) == (batch != 33)
     torch.manual_seed(7)
     pre = () if batch is None else (batch,)
     a = torch.randn(*pre, *((k, m) if a_mn else (m, k)), device="cuda", dtype=torch.bfloat16)
@@ -116,8 +118,22 @@ def test_gemm_by_pairs(a_mn, b_mn, m, n, k, batch):
     assert _rel_err(G.gemm(a, b, epilogue=G.EPI_RELU2_BWD, aux=aux, **kw), ref * 2 * aux.float().sqrt()) < 1e-2
 
 
+@pytest.mark.parametrize("m,n,k,element_bytes,pairs", [
+    (49152, 3072, 768, 2, True), (49152, 768, 3072, 2, True), (16384, 4096, 1536, 1, True),                       # 162, 174 us; 165, 173; 128, 140
+    (49152, 3072, 256, 2, False), (49152, 5120, 384, 2, False), (49152, 1536, 512, 2, False),                     # 119, 90; 190, 169; 76, 72
+    (49152, 50304, 768, 1, False), (16384, 50304, 768, 1, False), (49152, 768, 1024, 1, False)])                  # 2552, 1906; 726, 636; 46, 42
+def test_pairs_only_where_they_are_faster(m, n, k, element_bytes, pairs):
+    """Sizes at which both were timed (pairs, single CTAs): tiles of a few stages of K are not for pairs."""
+    from ml_experiments_b200.ops.runtime import ops
+
+    assert ops().gemm_by_pairs(m, n, k, 1, False, element_bytes, 1) == pairs
+
+
 def test_gemm_fp8_by_pairs():
     from ml_experiments_b200.ops.gemm import gemm
+    from ml_experiments_b200.ops.runtime import ops
+
+    assert ops().gemm_by_pairs(3000, 5008, 1424, 1, False, 1, 1)
 
     torch.manual_seed(8)
     m, n, k = 3000, 5008, 1424
