@@ -1133,13 +1133,22 @@ std::vector<Tensor> gpt_block_fwd(const Tensor& x, const Tensor& x0, const OptT&
   return out;
 }
 
-// gradients of x_a, of the first and of the second matrix
+// The way back through a projection x w^T from the gradient d of its result: gradients of its input (of relu^2's, where x is its result) and
+// of w. Called by itself where somebody waits for the latter; the two operators below then take the former as `done`.
+std::tuple<Tensor, Tensor> gpt_proj_bwd(const Tensor& d, const Tensor& x, const Tensor& w, bool relu2, const OptT& d_w, int64_t split, const Tensor& status) {
+  const c10::cuda::CUDAGuard guard(d.device());
+  Tensor dx = relu2 ? product(d, w, true, status, b200::EPI_RELU2_BWD, x) : product(d, w, true, status);
+  return {dx, weight_grad(d, x, d_w, split, status)};
+}
+
+// gradients of x_a, of the first and of the second matrix (undefined, as an empty tensor, where that is `done`)
 std::tuple<Tensor, Tensor, Tensor> gpt_mlp_bwd(const Tensor& dx, const Tensor& x_a, const Tensor& xn2, const Tensor& h, const Tensor& fc_w,
                                                const Tensor& out_w, const OptT& d_fc, const OptT& d_out, int64_t split_fc, int64_t split_out,
-                                               double eps, const Tensor& status) {
+                                               double eps, const Tensor& status, const OptT& done) {
   const c10::cuda::CUDAGuard guard(dx.device());
-  Tensor dpre = product(dx, out_w, true, status, b200::EPI_RELU2_BWD, h);
-  Tensor g_out = weight_grad(dx, h, d_out, split_out, status);
+  Tensor dpre, g_out;
+  if (done.has_value()) dpre = *done, g_out = at::empty({0}, dx.options());
+  else std::tie(dpre, g_out) = gpt_proj_bwd(dx, h, out_w, true, d_out, split_out, status);
   Tensor dxn2 = product(dpre, fc_w, true, status);
   Tensor g_fc = weight_grad(dpre, xn2, d_fc, split_fc, status);
   Tensor dx_a = at::empty_like(x_a);
@@ -1153,12 +1162,14 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> gpt_attn_bwd(const Tensor& dx_a, cons
                                                         const Tensor& proj_w, const Tensor& attn_lam, const OptT& ve, const Tensor& cos,
                                                         const Tensor& sin, const Tensor& doc_start, const Tensor& doc_end, Tensor dq, Tensor dlam,
                                                         const OptT& d_qkv, const OptT& d_proj, int64_t split_qkv, int64_t split_proj, int64_t H,
-                                                        int64_t D, double scale, int64_t window, double eps, const Tensor& status) {
+                                                        int64_t D, double scale, int64_t window, double eps, const Tensor& status,
+                                                        const OptT& done) {
   const c10::cuda::CUDAGuard guard(dx_a.device());
   const int64_t T = dx_a.size(0);
   TORCH_CHECK(dq.is_cuda() && dq.is_contiguous() && dq.scalar_type() == at::kFloat && dq.numel() == T * H * D, "dq: dense fp32 [T, H, D]");
-  Tensor dy = product(dx_a, proj_w, true, status);
-  Tensor g_proj = weight_grad(dx_a, y.view({T, H * D}), d_proj, split_proj, status);
+  Tensor dy, g_proj;
+  if (done.has_value()) dy = *done, g_proj = at::empty({0}, dx_a.options());
+  else std::tie(dy, g_proj) = gpt_proj_bwd(dx_a, y.view({T, H * D}), proj_w, false, d_proj, split_proj, status);
   C10_CUDA_CHECK(cudaMemsetAsync(dq.data_ptr(), 0, dq.numel() * sizeof(float), cur_stream()));
   Tensor dk = at::empty_like(y), dv = at::empty_like(y), delta = at::empty_like(lse);
   const Tensor q = qkvp.view({T, 3, H, D});
@@ -1198,8 +1209,9 @@ TORCH_LIBRARY(b200, m) {
   m.def("norm_bwd_add(Tensor dy, Tensor x, Tensor? dres, Tensor(a!) out, float eps) -> ()");
   m.def("mix_bwd(Tensor dmix, Tensor x, Tensor x0, Tensor? skip, Tensor lam, Tensor? skip_w, Tensor(a!) dx, Tensor(b!)? dskip, Tensor(c!) dx0_acc, Tensor(d!) dlam, Tensor(e!)? dskip_w, Tensor? dx_add=None) -> ()");
   m.def("gpt_block_fwd(Tensor x, Tensor x0, Tensor? skip, Tensor? skip_w, Tensor lam, Tensor? qkv_w, Tensor? attn_lam, Tensor? ve, Tensor? cos, Tensor? sin, Tensor? proj_w, Tensor fc_w, Tensor out_w, Tensor doc_start, Tensor doc_end, int H, int D, float scale, int window, float eps, Tensor status) -> Tensor[]");
-  m.def("gpt_mlp_bwd(Tensor dx, Tensor x_a, Tensor xn2, Tensor h, Tensor fc_w, Tensor out_w, Tensor(a!)? d_fc, Tensor(b!)? d_out, int split_fc, int split_out, float eps, Tensor status) -> (Tensor, Tensor, Tensor)");
-  m.def("gpt_attn_bwd(Tensor dx_a, Tensor x_mix, Tensor xn, Tensor qkv, Tensor qkvp, Tensor y, Tensor lse, Tensor qkv_w, Tensor proj_w, Tensor attn_lam, Tensor? ve, Tensor cos, Tensor sin, Tensor doc_start, Tensor doc_end, Tensor(a!) dq, Tensor(b!) dlam, Tensor(c!)? d_qkv, Tensor(d!)? d_proj, int split_qkv, int split_proj, int H, int D, float scale, int window, float eps, Tensor status) -> (Tensor, Tensor, Tensor, Tensor)");
+  m.def("gpt_mlp_bwd(Tensor dx, Tensor x_a, Tensor xn2, Tensor h, Tensor fc_w, Tensor out_w, Tensor(a!)? d_fc, Tensor(b!)? d_out, int split_fc, int split_out, float eps, Tensor status, Tensor? done=None) -> (Tensor, Tensor, Tensor)");
+  m.def("gpt_proj_bwd(Tensor d, Tensor x, Tensor w, bool relu2, Tensor(a!)? d_w, int split, Tensor status) -> (Tensor, Tensor)");
+  m.def("gpt_attn_bwd(Tensor dx_a, Tensor x_mix, Tensor xn, Tensor qkv, Tensor qkvp, Tensor y, Tensor lse, Tensor qkv_w, Tensor proj_w, Tensor attn_lam, Tensor? ve, Tensor cos, Tensor sin, Tensor doc_start, Tensor doc_end, Tensor(a!) dq, Tensor(b!) dlam, Tensor(c!)? d_qkv, Tensor(d!)? d_proj, int split_qkv, int split_proj, int H, int D, float scale, int window, float eps, Tensor status, Tensor? done=None) -> (Tensor, Tensor, Tensor, Tensor)");
   m.def("gpt_mix_bwd(Tensor dx_mix, Tensor x, Tensor x0, Tensor? skip, Tensor lam, Tensor? skip_w, Tensor(a!) dx0_acc, Tensor(b!) dlam, Tensor(c!)? dskip_w, Tensor? dx_add) -> (Tensor, Tensor)");
   m.def("qkv_post_fwd(Tensor qkv, Tensor? ve, Tensor lam, Tensor cos, Tensor sin, Tensor(a!) out, int H, int D, float eps) -> ()");
   m.def("qkv_post_bwd(Tensor dq, Tensor dk, Tensor dv, Tensor qkv, Tensor? ve, Tensor lam, Tensor cos, Tensor sin, Tensor(a!) dqkv, Tensor(b!)? dve, Tensor(c!) dlam, int H, int D, float eps) -> ()");
@@ -1272,6 +1284,7 @@ TORCH_LIBRARY_IMPL(b200, CUDA, m) {
   m.impl("gemm", &gemm);
   m.impl("gpt_block_fwd", &gpt_block_fwd);
   m.impl("gpt_mlp_bwd", &gpt_mlp_bwd);
+  m.impl("gpt_proj_bwd", &gpt_proj_bwd);
   m.impl("gpt_attn_bwd", &gpt_attn_bwd);
   m.impl("gpt_mix_bwd", &gpt_mix_bwd);
   m.impl("attn_fwd", &attn_fwd);

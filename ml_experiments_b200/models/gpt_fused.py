@@ -26,7 +26,7 @@ class _Saved:
 
 
 # Kernels of the operators that issue a block's (``runtime`` counts one a call).
-_BLOCK_FWD, _BLOCK_FWD_ATTN, _MLP_BWD, _ATTN_BWD = 4, 8, 5, 8
+_BLOCK_FWD, _BLOCK_FWD_ATTN, _PROJ_BWD, _MLP_BWD, _ATTN_BWD = 4, 8, 2, 5, 8
 
 
 def _wgrad(dy: Tensor, x: Tensor, out_shape, out: Tensor | None = None) -> Tensor:
@@ -139,6 +139,15 @@ def _forward_backward(model, input_seq: Tensor, target_seq: Tensor, swb: int, ne
         if hook is not None:
             hook(p, grads[id(p)])
 
+    def proj_bwd(p, d, x, relu2=False):
+        # a projection whose gradient somebody waits for comes back before the rest of its half of the block is issued
+        if id(p) not in grad_hooks:
+            return None
+        dx, g = o.gpt_proj_bwd(d, x, w16(p), relu2, out_buf(p), G.auto_split_k(*p.shape, T), st)
+        add_launches(_PROJ_BWD - 1)
+        put(p, g)
+        return dx
+
     if head.use_fp8:
         dxf = G.gemm(gl, w8, b_mn=True, alpha=1.0 / (grad_s * head.w_s))
         put(head.weight, G.gemm(gl, x8, a_mn=True, b_mn=True, out=out_buf(head.weight), out_dtype=torch.float32,
@@ -163,10 +172,12 @@ def _forward_backward(model, input_seq: Tensor, target_seq: Tensor, swb: int, ne
         if i in dskips:
             dx = dx + dskips.pop(i)
         fc, pj = blk.mlp.c_fc.weight, blk.mlp.c_proj.weight
+        done = proj_bwd(pj, dx, s.h, relu2=True)
         dx_a, g_fc, g_pj = o.gpt_mlp_bwd(dx, s.x_a, s.xn2, s.h, w16(fc), w16(pj), out_buf(fc), out_buf(pj), G.auto_split_k(*fc.shape, T),
-                                         G.auto_split_k(*pj.shape, T), EPS, st)
-        add_launches(_MLP_BWD - 1)
-        put(pj, g_pj)
+                                         G.auto_split_k(*pj.shape, T), EPS, st, done)
+        add_launches(_MLP_BWD - 1 - (0 if done is None else _PROJ_BWD))
+        if done is None:
+            put(pj, g_pj)
         put(fc, g_fc)
         if blk.attn is not None:
             a = blk.attn
@@ -176,12 +187,14 @@ def _forward_backward(model, input_seq: Tensor, target_seq: Tensor, swb: int, ne
             vi = ve_map[i]
             ve = ves[vi] if vi is not None else None
             dlam = gains[4 * i:4 * i + 2]
+            done = proj_bwd(wo, dx_a, s.y.view(T, HD))
             dx_mix, dve, g_wq, g_wo = o.gpt_attn_bwd(
                 dx_a, s.x_mix, s.xn, s.qkv, s.qkvp, s.y, s.lse, w16(wq).view(3 * HD, C), w16(wo), a.lambdas, ve, cos, sin, doc_start, doc_end,
                 dq_acc, dlam, out_buf(wq), out_buf(wo), G.auto_split_k(3 * HD, C, T), G.auto_split_k(C, HD, T), H, D, a.attn_scale, windows[i],
-                EPS, st)
-            add_launches(_ATTN_BWD - 1)
-            put(wo, g_wo)
+                EPS, st, done)
+            add_launches(_ATTN_BWD - 1 - (0 if done is None else _PROJ_BWD))
+            if done is None:
+                put(wo, g_wo)
             put(a.lambdas, dlam)
             if ve is not None:
                 # a value embedding feeds several layers: the first gradient waits for the next one and the two are

@@ -98,6 +98,35 @@ def test_loss_and_grad_equals_backward_of_the_loss():
         assert (m.get_parameter(n).grad.float() - 2 * want[n].float()).norm() <= 1e-2 * (2 * want[n].float()).norm() + 1e-8, n
 
 
+def test_gradient_hooks_are_called_before_the_rest_of_the_block_is_issued():
+    """A hook hands a finished gradient over (to a collective, say): that of an output projection comes before its half of the block goes on:
+    that of the MLP 3 kernels earlier, of the attention 6."""
+    from ml_experiments_b200.ops.runtime import launch_count
+
+    m = _model(False)
+    t = 1024
+    x, y = torch.randint(0, 50257, (t,), device="cuda"), torch.randint(0, 50257, (t,), device="cuda")
+    m.loss_and_grad(x, y, 2)
+    before = launch_count()
+    m.loss_and_grad(x, y, 2)
+    all_launches = launch_count() - before
+    want = {n: p.grad.clone() / 2 for n, p in m.named_parameters()}
+    called = {}
+    m._grad_hooks = {id(p): lambda p, g, n=n: called.update({n: (launch_count(), g)}) for n, p in m.named_parameters() if p.dim() > 1}
+    m.zero_grad(set_to_none=True)
+    before = launch_count()
+    m.loss_and_grad(x, y, 2)
+    assert launch_count() - before == all_launches
+    for i, blk in enumerate(m.blocks):
+        at = {n[9:]: c[0] for n, c in called.items() if n.startswith(f"blocks.{i}.")}
+        assert at["mlp.c_fc.weight"] - at["mlp.c_proj.weight"] == 3
+        if blk.attn is not None:
+            assert at["attn.qkv_w"] - at["attn.c_proj.weight"] >= 6        # and the scatter of a value embedding
+    for n, p in m.named_parameters():
+        if p.dim() > 1:
+            assert called[n][1].shape == p.shape and torch.allclose(called[n][1].float(), want[n].float(), rtol=5e-2, atol=2e-3 * want[n].abs().max().item()), n
+
+
 def test_muon_momentum_survives_a_state_dict_round_trip():
     """A momentum buffer restored from a checkpoint is moved into the optimizer's stacked buffer before the next step."""
     from ml_experiments_b200.optim import Muon
