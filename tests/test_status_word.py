@@ -65,4 +65,4 @@ def test_register_splits_are_checked_against_what_the_block_was_launched_with():
     assert fits(168, 384, need) and fits(161, 384, need)          # registers are handed out 8 a thread
     assert not fits(160, 384, need) and not fits(128, 384, need)
     source = (Path(__file__).resolve().parent.parent / "ml_experiments_b200" / "csrc" / "attn" / "attn_sm100.cu").read_text()
-    assert source.index("register_split_fits(attr.numRegs") < source.index("kern<<<grid, FWD_THREADS")
+    assert source.index("register_split_fits(attr.numRegs") < source.index("launch_early(kern, grid, FWD_THREADS")
