@@ -559,7 +559,7 @@ attn_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   uint64_t* bar_dq = bars + 3;     // dQ of a tile is in TMEM
   uint64_t* bar_sfree = bars + 4;  // S / dP of a tile are in registers, one arrival per compute warp
   uint64_t* bar_pds = bars + 5;    // P / dS of a tile are in place, one arrival per compute warp
-  uint64_t* bar_dqfree = bars + 6; // dQ of a tile is in registers, one arrival per compute warp
+  uint64_t* bar_dqfree = bars + 6; // dQ of a tile is in registers, one arrival per drain warp
   uint64_t* bar_q = bars + 7;      // [3] a Q / dO buffer is full
   uint64_t* bar_qe = bars + 10;    // [3] and empty again
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);

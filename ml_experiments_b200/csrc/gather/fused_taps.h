@@ -8,7 +8,9 @@
 //   w = lerp(kern, |rel| / max_rec) * (1 + |rel|/L)^(-expo) * valid,   out += w * bilinear(x, clamp(p, 0, L - 1.001))
 //   freq, phase : fp32 [B][L][H];  kern : fp32 [B][L][H][K];  expo : fp32 [B][L]
 //   backward: dx (fp32, atomics, zero it first), dfreq, dphase [B][L][H], dkern [B][L][H][K], dexpo_h [B][L][H]
-//   (the caller sums dexpo_h over heads). Most calls go to tele_band.h instead; these take head_dim 8, little work and very long strides.
+//   (the caller sums dexpo_h over heads). Most calls go to tele_band.h instead; these take what that refuses: head_dim 8, rows of less than
+//   64 channels, tables of more than 64 values, fewer than 128 or more than 32768 tokens, half above 119 or 120, operands off the 16-byte
+//   boundary, very long strides, and whatever is faster here (`tele_band_takes` estimates both).
 //
 // adaptive local conv (adaptive_local_conv.py:75-169, triton_adaptive_conv.py:81-318):
 //   s in [-half, half]:  r = |s| / half_w,  p = l + center + s,  valid = 0 <= p < L,
