@@ -1066,20 +1066,23 @@ bool tele_band_takes(const void* x, const void* y, int B, int L, int H, int D, i
   if ((long long)B * H * ((L + STEP - 1) / STEP) >= (1ll << 31)) return false;
   // The band grows with the strides, of which max_rec / half is the bound that the caller knows; the gather does not.
   if (!(max_rec > 0.f) || max_rec > (D == 16 ? 22.f : D == 32 ? 32.f : 48.f) * half) return false;
-  // What is left by estimates of both times in us, fitted to 1896 calls of 128 to 16384 tokens, 1 to 8 heads, tables of 4 to 64 values, strides up
-  // to 16 (10 to 14 % off, root mean square). A gather takes the taps of a row one after the other, or the time of all rows' taps where there are
-  // many; a band as many rounds as there are blocks of 128 rows for 148 multiprocessors, each of its steps of 64 keys, taps and table values
-  // (a table of no multiple of four is read value by value). Of these and 1400 others, 13 that go to the band are more than 3 % slower there,
-  // by 16 % at most; all take 0.73 (forward) and 0.79 of the gather's time on average. Gather and band, backward: 8 x 16384 x 4 heads of 64, table of 64
-  // 10130, 4300 us; 1200 tokens, a head of 128, 33 62, 105; 6000 x 4 of 16, 33 142, 208.
-  const int w = D == 16 ? 0 : D == 32 ? 1 : D == 64 ? 2 : 3;
-  static constexpr double TAP[2][4] = {{0.48, 0.36, 0.30, 0.31}, {0.63, 0.53, 0.47, 0.36}}, ROW_TAP[2][4] = {{13e-6, 19e-6, 34e-6, 63e-6}, {35e-6, 51e-6, 92e-6, 173e-6}};
-  static constexpr double KEYS[2][4] = {{0.60, 0.60, 0.62, 0.90}, {1.75, 1.80, 1.95, 2.15}};
-  const double taps = 2 * half + 1, rows = (double)B * L * H, steps = fmin(128 + 2.0 * max_rec, L) / STEP;
-  const double rounds = fmax(1.0, (double)B * H * ((L + ROWS - 1) / ROWS) / 148 * (backward ? 1.05 : half > 118 ? 1.25 : 1.0));   // (above: one block fits)
-  const double gather = (backward ? 19.0 : 6.5) + fmax(TAP[backward][w] * taps, ROW_TAP[backward][w] * rows * taps);
-  const double band = backward ? 25.5 + rounds * (KEYS[1][w] * steps + 0.145 * taps + (K % 4 ? 0.387 : 0.215) * K) : 11.5 + rounds * (KEYS[0][w] * steps + 0.06 * taps + 0.012 * K);
-  return 1.1 * band < gather;
+  // What is left by estimates of both times in us, fitted to some 3300 calls of 128 to 20000 tokens, 1 to 16 heads, tables of 2 to 64 values, strides
+  // up to 48 (10 to 12 % off, root mean square). A gather takes the taps of a row one after the other, or the time of all rows' taps where there
+  // are many. So does a band with its steps of 64 keys, taps and table values: one block of 128 rows, or all of them on 148 multiprocessors
+  // (a table of no multiple of four is read value by value). The faster way is missed by 1 to 2 % on average, and among calls of 300 us and more
+  // by 23 % at most. Gather and band, backward: 8 x 16384 x 4 heads of 64, table of 64 10130, 4300 us; 1200 tokens, a head of 128, 33 62, 105;
+  // 8 x 16384 x 4 of 16, 16 3770, 3350; 6000 x 4 of 16, 33 142, 208.
+  const int w = D == 16 ? 0 : D == 32 ? 1 : D == 64 ? 2 : 3, bk = backward;
+  static constexpr double START[2][4] = {{7.2, 7.9, 7.8, 9.3}, {19.5, 20.9, 21.6, 23.4}}, TAP[2][4] = {{0.46, 0.34, 0.29, 0.22}, {0.60, 0.47, 0.40, 0.265}};
+  static constexpr double ROW_TAP[2][4] = {{12.4e-6, 18.7e-6, 33e-6, 61.2e-6}, {34.4e-6, 50.1e-6, 90e-6, 169e-6}};
+  static constexpr double ONE_KEYS[2][4] = {{0.70, 0.70, 0.70, 1.0}, {2.15, 2.15, 2.15, 2.4}}, ALL_KEYS[2][4] = {{0.49, 0.51, 0.54, 0.72}, {1.62, 1.61, 1.69, 2.08}};
+  static constexpr double ALL_TABLE[2][4] = {{0.062, 0.062, 0.066, 0.09}, {0.36, 0.38, 0.42, 0.52}};
+  const double taps = 2 * half + 1, rows = (double)B * L * H, steps = fmin(128 + 2.0 * max_rec, L) / STEP, table = backward && K % 4 ? 1.8 * K : K;
+  const double share = (double)B * H * ((L + ROWS - 1) / ROWS) / 148 * (!backward && half > 118 ? 1.25 : 1.0);      // (above: one block at a time)
+  const double gather = START[bk][w] + fmax(TAP[bk][w] * taps, ROW_TAP[bk][w] * rows * taps);
+  const double one = ONE_KEYS[bk][w] * steps + (backward ? 0.09 * taps + 0.14 * table : 0.04 * taps + 0.005 * table);
+  const double all = share * (ALL_KEYS[bk][w] * steps + (backward ? 0.156 : 0.057) * taps + ALL_TABLE[bk][w] * table);
+  return 1.03 * ((backward ? 27.0 : 12.5) + fmax(one, all)) < gather;
 }
 
 void tele_band_fwd(const void* x, const float* freq, const float* phase, const float* kern, const float* expo, void* out, int B, int L, int H,
