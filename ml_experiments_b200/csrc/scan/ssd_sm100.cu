@@ -68,7 +68,7 @@ ssd_fwd_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
 
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   // Rounded up through an integer, so that accesses are generic ones: where the compiler sees shared memory it puts the masked decays and
-  // weights of a row (j < tid, below) behind a branch each. 8 x 4096, 32 heads of 64, state 64: 0.248 ms, by an offset 0.482.
+  // weights of a row (j < tid, below) behind a branch each. 8 x 4096, state 64, 32 heads of 64 and 6 of 128: 0.296, 0.247 ms, by an offset 0.532, 0.482.
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sC = smem;
   uint8_t* sB = sC + C_BYTES;
